@@ -65,10 +65,12 @@ def algorithmic_bytes(name, acq, hits_per_angle, band):
         "cap_cols": F * F * 8 + F * F * 10,
     }
     per_volume = {
-        # the gather with the z pass: cap cells in, the z-transformed spectrum and the OTF out
-        "gather": hits_per_angle * acq.nb_holo * 10 + D ** 3 * 8 + D ** 3,
-        "ypass": 2 * D ** 3 * 8,
-        "xpass": D ** 3 * 8 + 2 * D ** 3 * 4,
+        # cap cells in, the band planes of the spectrum and of the OTF out
+        "gather": hits_per_angle * acq.nb_holo * 10 + band * D * D * 9,
+        # the x and y passes run on the band planes, in place; the z pass widens them to the two volumes
+        "xpass": 2 * band * D * D * 8,
+        "ypass": 2 * band * D * D * 8,
+        "zpass": band * D * D * 8 + 2 * D ** 3 * 4,
     }
     return per_angle, per_volume
 
@@ -88,7 +90,7 @@ STAGE_KERNELS = {
     "fields": ("field_rows", "field_cols", "volkov_rows", "volkov_cols", "volkov_integ_rows",
                "volkov_integ_cols", "aber_fit", "form"),
     "cap_mapping": ("cap_rows", "cap_cols"),
-    "volume": ("gather", "ypass", "xpass"),
+    "volume": ("gather", "xpass", "ypass", "zpass"),
 }
 
 
@@ -137,7 +139,6 @@ def stage_roofline(acq, hits_per_angle, kern_ms, step_ms, peak):
 # workload's kernel is committed.
 NCU_TRAFFIC = {
     "extract_rows": (33.616128e6 + 0.341504e6, 0.0, "profiles/k_extract_rows_rytov_1024_64holos.md"),
-    "gather": (1083.210e6, 393.620e6, "profiles/k_gather_z_rytov_1024.md"),
 }
 
 
@@ -561,10 +562,10 @@ def cufft_reference(acq, kern):
                 "hologram_rows_16": round(ours("extract_rows") / n_chunks, 4),
                 "hologram_cols_16": round(ours("extract_cols") / n_chunks, 4),
                 "fields_2d_16": round(ours("field_rows", "field_cols") / n_chunks, 4),
-                "volume_3d": ours("gather", "ypass", "xpass")},
+                "volume_3d": ours("gather", "xpass", "ypass", "zpass")},
             "note": "the hand-written passes include their fused work (Tukey window, row packing and band "
                     "separation, crop, recentring, atan2/phasor, shifts, scaling and the index/absorption split; "
-                    "the volume's z pass runs inside the cap gather, so volume_3d includes the gather); "
+                    "volume_3d includes the cap gather); "
                     "the cuFFT calls are bare transforms"}
 
 

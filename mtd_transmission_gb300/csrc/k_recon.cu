@@ -13,13 +13,18 @@
 // Mapping (retroPropag_Born, src/fonctions.cpp:875-935) as a gather: voxel
 // column (X, Y) reads bin kx = (X - D/2) mod F for every angle whose cap window
 // covers it; each angle hits a column at most once, so the column's sums are
-// formed without atomics, in a fixed order; hit counts are exact (k_gather_z).
+// formed without atomics, in a fixed order; hit counts are exact (k_gather).
 //
 // Volume: fftshift3D, backward 3D FFT x Delta_f^3, fftshift3D, x -1/(2 n0 kv^2)
 // (main.cpp:282-352).  For even D the two shifts are sign modulations:
 //     out[m] = (-1)^(mx+my+mz+3D/2) IFFT3((-1)^(kx+ky+kz) V)[m].
-// The z pass runs inside the gather (k_gather_z); then a y pass, and an x pass
-// that writes the index and absorption volumes.
+// Caps reach only `band` of the D planes, and only the columns within F of the
+// centre, so the spectrum is kept as its band planes ([e][y][x], e = z - zmin)
+// and the transform along z comes last: the x and y passes run on band planes
+// only, and the z pass widens them to the D planes as it writes the index and
+// absorption volumes.  At 600 angles, 256^2 fields, 512^3 (band 220) the
+// stage moves 3.8 GB where transforming z first, over all columns, moved
+// 5.4 GB.
 #include "tdm_internal.cuh"
 #include "fft_warp.cuh"
 #include "form.cuh"
@@ -149,82 +154,110 @@ k_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, cons
 }
 
 // ---------------------------------------------------------------- cap accumulation
-// One warp per voxel column (X, Y); a CTA covers 32 consecutive X at one Y.
-// An angle's cap window is the F x F bins around its specular position, so a
-// column is covered by a fraction of the angles: the CTA first lists, in
-// ascending order, the angles whose window covers row Y and any of its 32
-// columns.  The lanes then take 32 consecutive listed angles at a time: each
-// lane loads its angle's cell plane in the column (a 2-byte record), and the
-// cap value only when the bin is a cap cell; the planes of the next two groups
-// and the values of the next group are loaded while the current one is
-// added, and groups without a hit are skipped.  An angle hits a column at
-// most once, at one plane, and
-// the column's running sums live in FP64 in shared memory.  When the group's
-// planes are distinct (seen through a plane -> lane ownership table) every
-// lane adds its own hit; otherwise lanes sharing a plane are grouped and the
-// group's lowest lane sums the members in ascending angle order (FP32, at
-// most 32 terms) before adding the sum.  The sums are deterministic, the hit
-// counts exact.  Widening the FP32 hits and narrowing the sums are done on
-// the integer pipe (fp_bits.cuh), so the FP64 pipe only adds.
+// One warp per voxel column (X, Y).  An angle's cap window is the F x F bins
+// around its specular position, so a column is covered by a fraction of the
+// angles: a CTA first lists, in ascending order, the angles whose window covers
+// its row Y and any of its columns.  The lanes then take 32 consecutive listed
+// angles at a time: each lane loads its angle's cell plane in the column (a
+// 2-byte record), and the cap value only when the bin is a cap cell; the
+// planes of the next two groups and the values of the next group are loaded
+// while the current one is added, and groups without a hit are skipped.  An
+// angle hits a column at most once, at one plane, and the column's running
+// sums live in FP64 in shared memory.  When the group's planes are distinct
+// (seen through a plane -> lane ownership table) every lane adds its own hit;
+// otherwise lanes sharing a plane are grouped and the group's lowest lane sums
+// the members in ascending angle order (FP32, at most 32 terms) before adding
+// the sum.  The sums are deterministic, the hit counts exact.  Widening the
+// FP32 hits and narrowing the sums are done on the integer pipe (fp_bits.cuh),
+// so the FP64 pipe only adds.
+
+// A listed angle: its specular x and its index.  Both fit 16 bits: an angle is
+// listed only when its window meets the CTA's columns, which bounds x by the
+// volume's side, and a stack has at most 65535 angles.
+struct Listed {
+    int16_t x;
+    uint16_t angle;
+};
 
 // Lists, in ascending order, the angles whose window covers row Y (by = Y -
-// D/2) and one of the columns bx0 .. bx0 + 31 of the CTA: list[i] = (posSpec
-// x, angle).  Returns the count; all NW warps of the CTA call it together.
+// D/2) and one of the columns bx0 .. bx0 + nx - 1 of the CTA.  Returns the
+// count; all NW warps of the CTA call it together, and it ends with a barrier.
+// 1024 angles a round: each warp tests its share in 32-angle pieces, and after
+// one barrier every warp scans the 32 pieces' ballots for the places of its own.
 template <int NW>
-__device__ __forceinline__ int list_angles(const int2* __restrict__ posspec, int M, int F, int by, int bx0, int2* list,
-                                           int* s_wc, int* s_listed) {
+__device__ __forceinline__ int list_angles(const int2* __restrict__ posspec, int M, int F, int by, int bx0, int nx,
+                                           Listed* list, unsigned (*s_bal)[32]) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x == 0) *s_listed = 0;
-    __syncthreads();
-    for (int a0 = 0; a0 < M; a0 += NW * 32) {
-        const int a = a0 + threadIdx.x;
-        int2 q = make_int2(0, 0);
-        bool keep = false;
-        if (a < M) {
-            q = posspec[a];
-            keep = (unsigned)(by + q.y) < (unsigned)F && bx0 + 31 + q.x >= 0 && bx0 + q.x < F;
+    constexpr int K = 32 / NW;  // pieces per warp and round
+    int base = 0;
+    for (int a0 = 0, r = 0; a0 < M; a0 += 1024, r ^= 1) {
+        int qx[K];
+        unsigned bal[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int a = a0 + (k * NW + w) * 32 + lane;
+            bool keep = false;
+            qx[k] = 0;
+            if (a < M) {
+                const int2 q = posspec[a];
+                keep = (unsigned)(by + q.y) < (unsigned)F && bx0 + nx - 1 + q.x >= 0 && bx0 + q.x < F;
+                qx[k] = q.x;
+            }
+            bal[k] = __ballot_sync(0xffffffffu, keep);
+            if (lane == 0) s_bal[r][k * NW + w] = bal[k];
         }
-        const unsigned bal = __ballot_sync(0xffffffffu, keep);
-        if (lane == 0) s_wc[w] = __popc(bal);
-        __syncthreads();
-        int off = *s_listed;
-        for (int k = 0; k < w; ++k) off += s_wc[k];
-        if (keep) list[off + __popc(bal & ((1u << lane) - 1u))] = make_int2(q.x, a);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int t = *s_listed;
-            for (int k = 0; k < NW; ++k) t += s_wc[k];
-            *s_listed = t;
+        __syncthreads();  // the other round's ballots are read before the barrier after next
+        const int own = __popc(s_bal[r][lane]);
+        int incl = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += t;
         }
-        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int off = base + __shfl_sync(0xffffffffu, incl - own, k * NW + w);
+            if ((bal[k] >> lane) & 1u)
+                list[off + __popc(bal[k] & ((1u << lane) - 1u))] =
+                    Listed{(int16_t)qx[k], (uint16_t)(a0 + (k * NW + w) * 32 + lane)};
+        }
+        base += __shfl_sync(0xffffffffu, incl, 31);
     }
-    return *s_listed;
+    __syncthreads();
+    return base;
 }
 
-// One warp sums column (bx, by) of the listed angles into acc / cnt (band
-// entries, zeroed here): the cells' planes and values are read from the cap
-// records at koff, the bin of the column in each angle's F x F window.
+// One warp sums column (bx, by) of the listed angles into acc (valid where cnt
+// is not 0) and cnt, band entries: the cells' planes and values are read from
+// the cap records at koff, the bin of the column in each angle's F x F window.
 __device__ __forceinline__ void gather_column(const float2* __restrict__ rec, const int16_t* __restrict__ recz,
-                                              const int2* list, int listed, size_t FF, size_t koff, int bx, int F,
+                                              const Listed* list, int listed, size_t FF, size_t koff, int bx, int F,
                                               int zmin, int band, double2* acc, uint16_t* cnt, uint8_t* own,
                                               float2* stg, int lane) {
-    for (int e = lane; e < band; e += 32) {
-        acc[e] = make_double2(0.0, 0.0);
-        cnt[e] = 0;
-    }
+    for (int e = lane; e < (band + 1) / 2; e += 32) reinterpret_cast<uint32_t*>(cnt)[e] = 0;
     // plane of listed angle i's cell in this column, or -1 when the angle's
     // window misses the column or the bin is outside its cap; the cap
     // value of a cell with plane z
     auto fetch_z = [&](int i) {
         int z = -1;
         if (i < listed) {
-            const int2 q = list[i];
-            if ((unsigned)(bx + q.x) < (unsigned)F) z = __ldg(&recz[(size_t)q.y * FF + koff]);
+            const Listed q = list[i];
+            if ((unsigned)(bx + q.x) < (unsigned)F) z = __ldg(&recz[(size_t)q.angle * FF + koff]);
         }
         return z;
     };
     auto fetch_v = [&](int i, int z) {
-        return z >= 0 ? __ldg(&rec[(size_t)list[i].y * FF + koff]) : make_float2(0.f, 0.f);
+        return z >= 0 ? __ldg(&rec[(size_t)list[i].angle * FF + koff]) : make_float2(0.f, 0.f);
+    };
+    // adds v to cell e's sums (a cell's first hit starts them) and k to its count
+    auto add = [&](int e, float2 v, int k) {
+        const unsigned n = cnt[e];
+        double2 t = make_double2(0.0, 0.0);
+        if (n) t = acc[e];
+        t.x += widen(v.x);
+        t.y += widen(v.y);
+        acc[e] = t;
+        cnt[e] = (uint16_t)(n + k);
     };
     int z_nxt = fetch_z(lane), z_nxt2 = fetch_z(32 + lane);
     float2 v_nxt = fetch_v(lane, z_nxt);
@@ -241,16 +274,10 @@ __device__ __forceinline__ void gather_column(const float2* __restrict__ rec, co
         __syncwarp();
         const bool shared_plane = e >= 0 && own[e] != lane;
         if (!__any_sync(0xffffffffu, shared_plane)) {
-            if (e >= 0) {
-                double2 t = acc[e];
-                t.x += widen(r.x);
-                t.y += widen(r.y);
-                acc[e] = t;
-                cnt[e]++;
-            }
+            if (e >= 0) add(e, r, 1);
         } else {
             const unsigned grp = __match_any_sync(0xffffffffu, e >= 0 ? e : -1 - lane);
-            stg[lane] = make_float2(r.x, r.y);
+            stg[lane] = r;
             __syncwarp();
             if (e >= 0 && (grp & ((1u << lane) - 1)) == 0) {  // lowest lane of its plane group
                 float sx = 0.0f, sy = 0.0f;
@@ -259,228 +286,225 @@ __device__ __forceinline__ void gather_column(const float2* __restrict__ rec, co
                     sx += u.x;
                     sy += u.y;
                 }
-                double2 t = acc[e];
-                t.x += widen(sx);
-                t.y += widen(sy);
-                acc[e] = t;
-                cnt[e] += (uint16_t)__popc(grp);
+                add(e, make_float2(sx, sy), __popc(grp));
             }
         }
         __syncwarp();
     }
 }
 
-// Cell (X, Y, zmin + e) of the normalised spectrum from its sums (main.cpp:243-249;
-// not normalised for the adjoint scatter); (-1)^(X+Y+Z) stands for the first
-// fftshift3D.
-__device__ __forceinline__ float2 gather_cell(const double2* acc, const uint16_t* cnt, int e, int X, int Y, int zmin,
-                                              int normalize, unsigned& n) {
-    n = cnt[e];
-    float2 val = make_float2(0.0f, 0.0f);
-    if (n) {
-        const double2 t = acc[e];
-        const float dn = normalize ? (float)n : 1.0f;  // FP32 division: FP64 division is a long sequence here
-        val = make_float2(narrow(t.x) / dn, narrow(t.y) / dn);
-    }
-    if ((X + Y + zmin + e) & 1) val = make_float2(-val.x, -val.y);
-    return val;
-}
+// k_gather: a CTA of kGW warps takes kGX consecutive columns at one Y, kGW at a
+// time, one per warp.  Each warp normalises its column's cells in place (not
+// normalised for the adjoint scatter; (-1)^(X+Y+Z) stands for the first
+// fftshift3D), and the CTA stores the kGW columns together as rows of
+// consecutive x (64-byte pieces) of the [e][y][x] spectrum, with the OTF mask
+// (Re != 0 after normalisation, main.cpp:262-267) and the counts, which one
+// column at a time would scatter plane by plane.  The grid covers the columns
+// that caps can reach; cells outside them and outside the band are cleared by
+// the host.
+//
+// Bound by issue and latency (FP64 sums in shared memory, dependent record
+// loads), so what counts is warps in flight: 4.2 KB of shared memory a warp at
+// a band of 220 planes.
+// 500 angles of 250^2, 512^3, all outputs: 528 us; with 16 columns' cells in a
+// tile beside the sums (72 KB a CTA) 575 us; the former kernel, which ran the z
+// transform too, 891 us.  64 angles of 512^2, 1024^3: 1.73, 3.66, 2.62 ms (the
+// empty blocks of 32 cells are skipped here).
+constexpr int kGW = 8, kGX = 16;
 
-// ---------------------------------------------------------------- gather fused with the z pass
-// k_gather_z: the cap gather and the inverse FFT along z (the first axis of
-// the 3D inverse FFT) in one kernel, so that the cap band (the planes of the
-// spectrum that caps reach) is neither written to HBM nor read back.  A CTA
-// of kGZ warps covers 32 consecutive columns (X) at one Y; a warp takes its
-// columns G = WarpFFT<D>::G at a time (the lanes of one column transform),
-// sums each with gather_column into its own FP64 sums, loads the G
-// normalised columns into registers (zero outside the band) and
-// inverse-transforms them along z together.  The transform's exchange
-// buffers (T (T + 1) slots per transform, fft_warp_regs_lean) overlay the
-// sums, which are in registers by then.  Each lane stores its outputs
-// directly (lane-minor order is contiguous in z) into the [y][x][z] volume.
-// The OTF mask (Re != 0 after normalisation, main.cpp:262-267) of the CTA's
-// 32 columns is collected as one bit per column and plane in shared memory
-// and stored as 32-byte rows; planes outside the band are cleared by the
-// host.
-constexpr int kGZ = 4;  // warps per CTA
-
-template <int D>
-struct GatherZ {
-    using W = WarpFFT<D>;
-    static constexpr int G = W::G, T = W::T, E = W::E;
-    static constexpr int COLS = 32 / kGZ;  // columns per warp
-    static_assert(COLS % G == 0, "a warp's columns split into groups of G");
-    // per-warp region: G sums (double2) and G counts (uint16) of the band, or,
-    // once the sums are in registers, the G exchange buffers
-    __host__ __device__ static size_t region(int band) {
-        const size_t sums = (size_t)G * band * (sizeof(double2) + sizeof(uint16_t));
-        const size_t xch = (size_t)G * T * (T + 1) * sizeof(float2);
-        return ((sums > xch ? sums : xch) + 15) & ~size_t(15);
-    }
-    __host__ __device__ static size_t own_bytes(int band) { return (size_t)((band + 15) & ~15); }
-    static size_t smem(int band, int n) {
-        return kGZ * (region(band) + 32 * sizeof(float2) + own_bytes(band)) + (((size_t)band * 4 + 7) & ~size_t(7)) +
-               (size_t)n * sizeof(int2);
+struct GatherSmem {
+    // per warp: sums, counts (uint16), plane owners (uint8) and a 32-lane
+    // staging row, at a pitch of 16 bytes mod 128: with the normalised cell of
+    // an odd plane in the upper half of its sums' slot, the CTA-wide store's
+    // reads (8 columns x 2 planes a half-warp) fall in distinct banks
+    __host__ __device__ static int cnt_at(int band) { return band * 16; }
+    __host__ __device__ static int own_at(int band) { return cnt_at(band) + ((band * 2 + 15) & ~15); }
+    __host__ __device__ static int stg_at(int band) { return own_at(band) + ((band + 15) & ~15); }
+    __host__ __device__ static int pitch(int band) { return ((stg_at(band) + 32 * 8 - 16 + 127) & ~127) + 16; }
+    __host__ __device__ static size_t bytes(int band, int n) {
+        return (size_t)kGW * pitch(band) + (size_t)n * sizeof(Listed);
     }
 };
 
-template <int D>
-__global__ void __launch_bounds__(kGZ * 32, 5)
-k_gather_z(const float2* __restrict__ rec, const int16_t* __restrict__ recz, const int2* __restrict__ posspec, int M,
-           Params p, const float2* __restrict__ tw, float2* __restrict__ vol, uint32_t* __restrict__ cnt_out,
-           uint8_t* __restrict__ otf, int normalize) {
-    using Z = GatherZ<D>;
-    constexpr int G = Z::G, T = Z::T, E = Z::E;
+__global__ void __launch_bounds__(kGW * 32)
+k_gather(const float2* __restrict__ rec, const int16_t* __restrict__ recz, const int2* __restrict__ posspec, int M,
+         Params p, float2* __restrict__ vol, uint32_t* __restrict__ cnt_out, uint8_t* __restrict__ otf,
+         int normalize) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    __shared__ int s_wc[kGZ];
-    __shared__ int s_listed;
-    const int band = p.band;
-    const size_t reg = Z::region(band), ownb = Z::own_bytes(band);
+    __shared__ unsigned s_bal[2][32];
+    const int band = p.band, F = p.F, D = p.D, h = D / 2, zmin = p.zmin;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    unsigned char* region = smraw + w * reg;
-    double2* acc0 = reinterpret_cast<double2*>(region);                  // G x band
-    uint16_t* cnt0 = reinterpret_cast<uint16_t*>(acc0 + G * band);      // G x band
-    float2* stg = reinterpret_cast<float2*>(smraw + kGZ * reg) + w * 32;
-    uint8_t* own = smraw + kGZ * (reg + 32 * sizeof(float2)) + w * ownb;
-    uint32_t* bits = reinterpret_cast<uint32_t*>(smraw + kGZ * (reg + 32 * sizeof(float2) + ownb));  // band
-    int2* list = reinterpret_cast<int2*>(reinterpret_cast<unsigned char*>(bits) + (((size_t)band * 4 + 7) & ~size_t(7)));
-    const int F = p.F, h = D / 2, zmin = p.zmin;
-    const size_t FF = (size_t)F * F;
-    const int Y = blockIdx.y, by = Y - h, X0 = blockIdx.x * 32;
-    if (otf)
-        for (int e = threadIdx.x; e < band; e += kGZ * 32) bits[e] = 0;  // ordered by list_angles' barriers
-    const int listed = list_angles<kGZ>(posspec, M, F, by, X0 - h, list, s_wc, &s_listed);
-    const int g = lane / T, j = lane % T;  // this lane's transform of the group, and its lane in it
-    for (int r = 0; r < Z::COLS / G; ++r) {
-#pragma unroll 1
-        for (int gg = 0; gg < G; ++gg) {
-            const int X = X0 + w + kGZ * (r * G + gg);
-            const int bx = X - h;
-            const size_t koff = (size_t)(((by % F) + F) % F) * F + ((bx % F) + F) % F;
-            double2* acc = acc0 + gg * band;
-            const uint16_t* cnt = cnt0 + gg * band;
-            gather_column(rec, recz, list, listed, FF, koff, bx, F, zmin, band, acc, cnt0 + gg * band, own, stg,
-                          lane);
-            // normalised cells, in place: cell e's float2 goes to bytes [8e, 8e + 8), over sums of cells
-            // below the current 32, which have been read (a rolled loop keeps the kernel's code small)
-            float2* cell = reinterpret_cast<float2*>(acc);
-            for (int e0 = 0; e0 < band; e0 += 32) {
-                const int e = e0 + lane;
-                float2 v = make_float2(0.f, 0.f);
-                if (e < band) {
-                    unsigned n;
-                    v = gather_cell(acc, cnt, e, X, Y, zmin, normalize, n);
-                    if (cnt_out) cnt_out[((size_t)(zmin + e) * D + Y) * D + X] = n;
-                    if (otf && v.x != 0.0f) atomicOr(&bits[e], 1u << (X - X0));
+    const int pitch = GatherSmem::pitch(band), cnt_at = GatherSmem::cnt_at(band);
+    unsigned char* mine = smraw + w * pitch;
+    double2* acc = reinterpret_cast<double2*>(mine);
+    uint16_t* cnt = reinterpret_cast<uint16_t*>(mine + cnt_at);
+    uint8_t* own = mine + GatherSmem::own_at(band);
+    float2* stg = reinterpret_cast<float2*>(mine + GatherSmem::stg_at(band));
+    Listed* list = reinterpret_cast<Listed*>(smraw + kGW * pitch);
+    auto cell = [](unsigned char* col, int e) { return reinterpret_cast<float2*>(col + e * 16 + (e & 1) * 8); };
+    const size_t FF = (size_t)F * F, plane = (size_t)D * D;
+    const int X0 = p.xa + blockIdx.x * kGX, Y = p.ya + blockIdx.y, by = Y - h;
+    const int listed = list_angles<kGW>(posspec, M, F, by, X0 - h, kGX, list, s_bal);
+    const int ky = ((by % F) + F) % F;
+    for (int c0 = 0; c0 < kGX; c0 += kGW) {
+        const int X = X0 + c0 + w, bx = X - h;
+        gather_column(rec, recz, list, listed, FF, (size_t)ky * F + ((bx % F) + F) % F, bx, F, zmin, band, acc, cnt,
+                      own, stg, lane);
+        for (int e0 = 0; e0 < band; e0 += 32) {
+            const int e = e0 + lane;
+            const unsigned n = e < band ? cnt[e] : 0;
+            float2 v = make_float2(0.f, 0.f);
+            if (__any_sync(0xffffffffu, n != 0)) {
+                if (n) {
+                    const double2 t = acc[e];
+                    const float dn = normalize ? (float)n : 1.0f;  // FP32 division: FP64 division is a long sequence here
+                    v = make_float2(narrow(t.x) / dn, narrow(t.y) / dn);
                 }
-                __syncwarp();
-                if (e < band) cell[e] = v;
+                if ((X + Y + zmin + e) & 1) v = make_float2(-v.x, -v.y);
             }
+            if (e < band) *cell(mine, e) = v;
         }
-        __syncwarp();
-        const int X = X0 + w + kGZ * (r * G + g);
-        const float2* cell = reinterpret_cast<const float2*>(acc0 + g * band);
-        float2 x[E];
-#pragma unroll
-        for (int n1 = 0; n1 < E; ++n1) {
-            const int e = j + n1 * T - zmin;
-            x[n1] = (unsigned)e < (unsigned)band ? cell[e] : make_float2(0.f, 0.f);
-        }
-        // the exchange buffers overlay the sums: every lane has read its column (the transform's first __syncwarp)
-        fft_warp_regs_lean<D, +1>(x, reinterpret_cast<float2*>(region) + g * T * (T + 1), j, tw);
-        float2* col = vol + ((size_t)Y * D + X) * D;
-#pragma unroll
-        for (int q = 0; q < E / T; ++q) {
-#pragma unroll
-            for (int k2 = 0; k2 < T; ++k2) col[j + q * T + E * k2] = x[q * T + k2];
-        }
-        __syncwarp();  // the next group's sums overlay the exchange buffers
-    }
-    if (otf) {
         __syncthreads();
-        uint8_t* o = otf + (size_t)Y * D + X0;
-        const size_t plane = (size_t)D * D;
-        if ((reinterpret_cast<uintptr_t>(otf) & 15) == 0) {
-            for (int i = threadIdx.x; i < 2 * band; i += kGZ * 32) {  // 16 columns' flags per store
-                const uint32_t b = bits[i >> 1] >> (16 * (i & 1));
-                uint32_t v[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const uint32_t nib = (b >> (4 * t)) & 0xFu;
-                    v[t] = (nib & 1u) | ((nib & 2u) << 7) | ((nib & 4u) << 14) | ((nib & 8u) << 21);
-                }
-                *reinterpret_cast<uint4*>(o + (size_t)(zmin + (i >> 1)) * plane + 16 * (i & 1)) =
-                    make_uint4(v[0], v[1], v[2], v[3]);
-            }
-        } else {
-            for (int i = threadIdx.x; i < 32 * band; i += kGZ * 32)
-                o[(size_t)(zmin + i / 32) * plane + i % 32] = (uint8_t)((bits[i / 32] >> (i % 32)) & 1u);
+        const int c = threadIdx.x % kGW;
+        unsigned char* col = smraw + c * pitch;
+        size_t o = (size_t)Y * D + X0 + c0 + c + (threadIdx.x / kGW) * plane;
+        for (int e = threadIdx.x / kGW; e < band; e += 32, o += 32 * plane) {
+            const float2 v = *cell(col, e);
+            vol[o] = v;
+            if (cnt_out) cnt_out[zmin * plane + o] = reinterpret_cast<uint16_t*>(col + cnt_at)[e];
+            if (otf) otf[zmin * plane + o] = v.x != 0.0f;
         }
+        if (c0 + kGW < kGX) __syncthreads();  // the next columns take the sums' place
     }
 }
 
+// ---------------------------------------------------------------- 3D FFT passes
+// Column passes (y, z): a CTA transforms B consecutive x.  The T threads of
+// a transform sit B apart, so a warp's lanes are consecutive x (of two
+// neighbouring elements): loads and stores go straight between registers and
+// global memory in 128-byte lines, and shared memory holds the FFT's one
+// transposing exchange only, with a CTA barrier around it.  (A warp per
+// transform, with the columns staged and unstaged through shared memory, took
+// three times the shared-memory traffic and bounded the passes.)  Bound by HBM:
+// 512^3 with a band of 220, x 137 us and y 144 us (6.7 and 6.4 TB/s), z 337 us
+// (4.5 TB/s, most of it stores); over all planes y and x took 405 and 432 us.
+// B = 8 leaves 32-byte pieces in the z pass's stores (713 us), B = 32 one CTA an
+// SM (y 182, z 352 us).
 template <int D>
-struct PassCfg {
+struct ColPass {
     using W = WarpFFT<D>;
-    static constexpr int B = 16;           // transforms per CTA
-    static constexpr int NT = B * W::T;    // threads per CTA
+    static constexpr int B = 16;
+    static constexpr int NT = B * W::T;
+    static constexpr size_t SMEM = (size_t)B * W::STRIDE * sizeof(float2);
+    static constexpr int CTAS = NT <= 128 ? 4 : NT <= 256 ? 2 : 1;  // 128 registers a thread
+};
+
+// Row pass (x): a warp per G rows, registers to registers.
+template <int D>
+struct RowPass {
+    using W = WarpFFT<D>;
+    static constexpr int B = 8 * W::G;
+    static constexpr int NT = 256;
     static constexpr size_t SMEM = (size_t)B * W::STRIDE * sizeof(float2);
 };
 
-// Inverse FFT along y, in place, for B consecutive z at fixed x.
+// FFT along x of the band planes' rows in [ya, yb), in place.  Inverse (DIR
+// +1): columns outside [xa, xb) hold nothing and are taken as zero.  Forward:
+// the last pass of the forward operator, x (-1)^(X+Y+Z), only [xa, xb) written.
 template <int D, int DIR>
-__global__ void __launch_bounds__(PassCfg<D>::NT)
-k_ypass(float2* __restrict__ vol, const float2* __restrict__ tw) {
-    using C = PassCfg<D>;
+__global__ void __launch_bounds__(RowPass<D>::NT, 2)
+k_xpass(float2* __restrict__ vol, const float2* __restrict__ tw, Params p) {
+    using C = RowPass<D>;
     using W = typename C::W;
-    constexpr int B = C::B, NT = C::NT;
+    constexpr int T = W::T, E = W::E;
     extern __shared__ float2 sm[];
-    const int tr = threadIdx.x / W::T, j = threadIdx.x % W::T;
-    const int z0 = blockIdx.x * B, X = blockIdx.y;
-#pragma unroll  // every load in flight before the first store (latency-bound at 8)
-    for (int r = 0; r < B * D / NT; ++r) {
-        const int i = threadIdx.x + r * NT, t = i % B, Y = i / B;
-        sm[t * W::STRIDE + W::pad(Y)] = vol[((size_t)Y * D + X) * D + z0 + t];
+    const int tr = threadIdx.x / T, j = threadIdx.x % T;
+    const int ny = p.yb - p.ya;
+    int r = blockIdx.x * C::B + tr;  // band row: plane e, row Y
+    const bool ok = r < p.band * ny;
+    if (!ok) r = 0;
+    const int e = r / ny, Y = p.ya + r % ny;
+    float2* row = vol + ((size_t)e * D + Y) * D;
+    float2 x[E];
+#pragma unroll
+    for (int n1 = 0; n1 < E; ++n1) {
+        const int X = j + n1 * T;
+        x[n1] = DIR < 0 || (X >= p.xa && X < p.xb) ? row[X] : make_float2(0.f, 0.f);
     }
-    __syncthreads();
-    fft_warp<D, DIR>(sm + tr * W::STRIDE, j, tw);
-    __syncthreads();
-#pragma unroll 8
-    for (int r = 0; r < B * D / NT; ++r) {
-        const int i = threadIdx.x + r * NT, t = i % B, Y = i / B;
-        vol[((size_t)Y * D + X) * D + z0 + t] = sm[t * W::STRIDE + W::pad(Y)];
+    fft_warp_regs<D, DIR>(x, sm + tr * W::STRIDE, j, tw);
+    if (!ok) return;
+    const float sg = DIR < 0 && ((j + Y + p.zmin + e) & 1) ? -1.0f : 1.0f;  // X has j's parity
+#pragma unroll
+    for (int q = 0; q < E / T; ++q) {
+#pragma unroll
+        for (int k2 = 0; k2 < T; ++k2) {
+            const int X = j + q * T + E * k2;
+            const float2 v = x[q * T + k2];
+            if (DIR > 0) row[X] = v;
+            else if (X >= p.xa && X < p.xb) row[X] = make_float2(v.x * sg, v.y * sg);
+        }
     }
 }
 
-// Inverse FFT along x for B consecutive z at fixed y, scaled and sign-modulated,
-// written as the index (real) and absorption (imaginary) volumes, x fastest.
-template <int D>
-__global__ void __launch_bounds__(PassCfg<D>::NT)
-k_xpass(const float2* __restrict__ vol, const float2* __restrict__ tw, float scale, int zblock0, float* __restrict__ re,
-        float* __restrict__ im) {
-    using C = PassCfg<D>;
+// FFT along y of the band planes, in place; inverse: rows outside [ya, yb)
+// are taken as zero; forward: only rows in [ya, yb) are written.
+template <int D, int DIR>
+__global__ void __launch_bounds__(ColPass<D>::NT, ColPass<D>::CTAS)
+k_ypass(float2* __restrict__ vol, const float2* __restrict__ tw, Params p) {
+    using C = ColPass<D>;
     using W = typename C::W;
-    constexpr int B = C::B, NT = C::NT;
+    constexpr int T = W::T, E = W::E;
     extern __shared__ float2 sm[];
-    const int tr = threadIdx.x / W::T, j = threadIdx.x % W::T;
-    const int z0 = (zblock0 + blockIdx.x) * B, Y = blockIdx.y;
-#pragma unroll  // every load in flight before the first store (latency-bound at 8)
-    for (int r = 0; r < B * D / NT; ++r) {
-        const int i = threadIdx.x + r * NT, t = i % B, X = i / B;
-        sm[t * W::STRIDE + W::pad(X)] = vol[((size_t)Y * D + X) * D + z0 + t];
+    const int t = threadIdx.x % C::B, j = threadIdx.x / C::B;
+    float2* col = vol + (size_t)blockIdx.y * D * D + blockIdx.x * C::B + t;
+    float2 x[E];
+#pragma unroll
+    for (int n1 = 0; n1 < E; ++n1) {
+        const int Y = j + n1 * T;
+        x[n1] = DIR < 0 || (Y >= p.ya && Y < p.yb) ? col[(size_t)Y * D] : make_float2(0.f, 0.f);
     }
-    __syncthreads();
-    fft_warp<D, +1>(sm + tr * W::STRIDE, j, tw);
-    __syncthreads();
-    const int par = (3 * (D / 2)) & 1;
-#pragma unroll 8
-    for (int r = 0; r < B * D / NT; ++r) {
-        const int i = threadIdx.x + r * NT, t = i / D, X = i % D, Z = z0 + t;
-        const float2 v = sm[t * W::STRIDE + W::pad(X)];
-        const float sg = ((X + Y + Z + par) & 1) ? -scale : scale;
-        const size_t o = ((size_t)Z * D + Y) * D + X;
-        if (re) re[o] = v.x * sg;
-        if (im) im[o] = v.y * sg;
+    fft_cta_regs<D, DIR>(x, sm + t * W::STRIDE, j, tw);
+#pragma unroll
+    for (int q = 0; q < E / T; ++q) {
+#pragma unroll
+        for (int k2 = 0; k2 < T; ++k2) {
+            const int Y = j + q * T + E * k2;
+            if (DIR > 0 || (Y >= p.ya && Y < p.yb)) col[(size_t)Y * D] = x[q * T + k2];
+        }
+    }
+}
+
+// Inverse FFT along z of the band (zero elsewhere), scaled and
+// sign-modulated, written as the index (real) and absorption (imaginary)
+// volumes, x fastest, for rows y0 + blockIdx.y.
+template <int D>
+__global__ void __launch_bounds__(ColPass<D>::NT, ColPass<D>::CTAS)
+k_zpass(const float2* __restrict__ vol, const float2* __restrict__ tw, Params p, float scale, int y0,
+        float* __restrict__ re, float* __restrict__ im) {
+    using C = ColPass<D>;
+    using W = typename C::W;
+    constexpr int T = W::T, E = W::E;
+    extern __shared__ float2 sm[];
+    const int t = threadIdx.x % C::B, j = threadIdx.x / C::B;
+    const int X = blockIdx.x * C::B + t, Y = y0 + blockIdx.y;
+    const float2* col = vol + (size_t)Y * D + X;
+    float2 x[E];
+#pragma unroll
+    for (int n1 = 0; n1 < E; ++n1) {
+        const int e = j + n1 * T - p.zmin;
+        x[n1] = (unsigned)e < (unsigned)p.band ? col[(size_t)e * D * D] : make_float2(0.f, 0.f);
+    }
+    fft_cta_regs<D, +1>(x, sm + t * W::STRIDE, j, tw);
+    const float sg = ((X + Y + j + 3 * (D / 2)) & 1) ? -scale : scale;  // z has j's parity
+    const size_t o = (size_t)Y * D + X;
+#pragma unroll
+    for (int q = 0; q < E / T; ++q) {
+#pragma unroll
+        for (int k2 = 0; k2 < T; ++k2) {
+            const size_t z = j + q * T + E * k2;
+            if (re) re[z * D * D + o] = x[q * T + k2].x * sg;
+            if (im) im[z * D * D + o] = x[q * T + k2].y * sg;
+        }
     }
 }
 
@@ -491,65 +515,36 @@ k_xpass(const float2* __restrict__ vol, const float2* __restrict__ tw, float sca
 // is A = S G with G = T^-1 = M_in FFT3(M_out x) / (s D^3) and S the sampling
 // of each angle's cap cells (the cells the gather fills, same geometry); its
 // adjoint is A^H = G^H S^H, G^H = M_out IFFT3(M_in .) / (s D^3) and S^H the
-// unnormalised scatter, i.e. k_gather_z without the division by the hit
-// count, followed by the y and x passes with scale 1 / (s D^3).
+// unnormalised scatter, i.e. k_gather without the division by the hit
+// count, followed by the x, y and z passes with scale 1 / (s D^3).
 
-// Forward x pass: FFT along x of B consecutive z rows at fixed y of the
-// index/absorption volumes (x M_out x scale), into the [y][x][z] spectrum.
+// Forward z pass: FFT along z of the index/absorption volumes (x M_out x
+// scale), only the cap band written (the sampling reads nothing else).
 template <int D>
-__global__ void __launch_bounds__(PassCfg<D>::NT)
-k_fxpass(const float* __restrict__ re, const float* __restrict__ im, const float2* __restrict__ tw, float scale,
-         float2* __restrict__ vol) {
-    using C = PassCfg<D>;
+__global__ void __launch_bounds__(ColPass<D>::NT, ColPass<D>::CTAS)
+k_fzpass(const float* __restrict__ re, const float* __restrict__ im, const float2* __restrict__ tw, Params p,
+         float scale, float2* __restrict__ vol) {
+    using C = ColPass<D>;
     using W = typename C::W;
-    constexpr int B = C::B, NT = C::NT;
+    constexpr int T = W::T, E = W::E;
     extern __shared__ float2 sm[];
-    const int tr = threadIdx.x / W::T, j = threadIdx.x % W::T;
-    const int z0 = blockIdx.x * B, Y = blockIdx.y;
-    const int par = (3 * (D / 2)) & 1;
-#pragma unroll  // every load in flight before the first store
-    for (int r = 0; r < B * D / NT; ++r) {
-        const int i = threadIdx.x + r * NT, t = i / D, X = i % D, Z = z0 + t;
-        const size_t o = ((size_t)Z * D + Y) * D + X;
-        const float sg = ((X + Y + Z + par) & 1) ? -scale : scale;
-        sm[t * W::STRIDE + W::pad(X)] = make_float2(re[o] * sg, im ? im[o] * sg : 0.0f);
-    }
-    __syncthreads();
-    fft_warp<D, -1>(sm + tr * W::STRIDE, j, tw);
-    __syncthreads();
-#pragma unroll 8
-    for (int r = 0; r < B * D / NT; ++r) {
-        const int i = threadIdx.x + r * NT, t = i % B, X = i / B;
-        vol[((size_t)Y * D + X) * D + z0 + t] = sm[t * W::STRIDE + W::pad(X)];
-    }
-}
-
-// Forward z pass: FFT along z of B columns (all planes in), x M_in, only the
-// cap band written (the sampling reads nothing else).
-template <int D>
-__global__ void __launch_bounds__(PassCfg<D>::NT)
-k_fzpass(float2* __restrict__ vol, const float2* __restrict__ tw, int zmin, int band) {
-    using C = PassCfg<D>;
-    using W = typename C::W;
-    constexpr int B = C::B, T = W::T, E = W::E;
-    extern __shared__ float2 sm[];
-    const int t = threadIdx.x / T, j = threadIdx.x % T;
-    const size_t c = (size_t)blockIdx.x * B + t;  // y * D + x
-    const int XY = (int)(c % D) + (int)(c / D);
-    float2* col = vol + c * D;
+    const int t = threadIdx.x % C::B, j = threadIdx.x / C::B;
+    const int X = blockIdx.x * C::B + t, Y = blockIdx.y;
+    const size_t o = (size_t)Y * D + X;
+    const float sg = ((X + Y + j + 3 * (D / 2)) & 1) ? -scale : scale;  // z has j's parity
     float2 x[E];
 #pragma unroll
-    for (int n1 = 0; n1 < E; ++n1) x[n1] = col[j + n1 * T];
-    fft_warp_regs<D, -1>(x, sm + t * W::STRIDE, j, tw);
+    for (int n1 = 0; n1 < E; ++n1) {
+        const size_t z = j + n1 * T;
+        x[n1] = make_float2(re[z * D * D + o] * sg, im ? im[z * D * D + o] * sg : 0.0f);
+    }
+    fft_cta_regs<D, -1>(x, sm + t * W::STRIDE, j, tw);
 #pragma unroll
     for (int q = 0; q < E / T; ++q) {
 #pragma unroll
         for (int k2 = 0; k2 < T; ++k2) {
-            const int Z = j + q * T + E * k2;
-            if (Z >= zmin && Z < zmin + band) {
-                const float2 v = x[q * T + k2];
-                col[Z] = ((XY + Z) & 1) ? make_float2(-v.x, -v.y) : v;
-            }
+            const int e = j + q * T + E * k2 - p.zmin;
+            if ((unsigned)e < (unsigned)p.band) vol[(size_t)e * D * D + o] = x[q * T + k2];
         }
     }
 }
@@ -581,7 +576,7 @@ k_cap_sample(const float2* __restrict__ vol, const int2* __restrict__ posspec, P
         if (z >= 0) {
             const float2 d = data ? data[o] : make_float2(0.f, 0.f);
             const int X = cap_col(p, kx, ps.x), Y = cap_col(p, ky, ps.y);
-            v = vol[((size_t)Y * D + X) * D + z];
+            v = vol[((size_t)(z - p.zmin) * D + Y) * D + X];
             v = make_float2(v.x - d.x, v.y - d.y);
             m2 += (double)v.x * v.x + (double)v.y * v.y;
         }
@@ -783,6 +778,37 @@ static cudaError_t download_after(tdm_ctx* c, cudaStream_t st, cudaEvent_t ev, v
     return e;
 }
 
+// The gather of n angles' cap records into the band spectrum.
+int launch_gather(tdm_ctx* c, CapRecs rec, const int2* posspec, int n, uint32_t* cnt, uint8_t* otf, int normalize,
+                  cudaStream_t st) {
+    const Params& p = c->p;
+    const size_t smem = GatherSmem::bytes(p.band, n);
+    if (smem > kMaxSmemPerCta) return TDM_EUNSUPPORTED;
+    if (allow_smem(k_gather, smem)) return TDM_ECUDA;
+    Launch l(c, K_GATHER, st);
+    k_gather<<<dim3((p.xb - p.xa) / kGX, p.yb - p.ya), kGW * 32, smem, st>>>(rec.val, rec.z, posspec, n, p, c->b.vol,
+                                                                             cnt, otf, normalize);
+    return TDM_OK;
+}
+
+// x and y passes on the band planes, after the gather (DIR +1).
+template <int D>
+int launch_xy(tdm_ctx* c, cudaStream_t st) {
+    using R = RowPass<D>;
+    using P = ColPass<D>;
+    const Params& p = c->p;
+    if (allow_smem(k_xpass<D, 1>, R::SMEM) || allow_smem(k_ypass<D, 1>, P::SMEM)) return TDM_ECUDA;
+    {
+        Launch l(c, K_XPASS, st);
+        k_xpass<D, 1><<<(p.band * (p.yb - p.ya) + R::B - 1) / R::B, R::NT, R::SMEM, st>>>(c->b.vol, c->b.tw, p);
+    }
+    {
+        Launch l(c, K_YPASS, st);
+        k_ypass<D, 1><<<dim3(D / P::B, p.band), P::NT, P::SMEM, st>>>(c->b.vol, c->b.tw, p);
+    }
+    return TDM_OK;
+}
+
 template <int D>
 int volume_impl(tdm_ctx* c, int n, const VolumeOut& out, cudaStream_t st, CapRecs rec, const int2* posspec,
                 cudaEvent_t ev_gathered) {
@@ -790,37 +816,30 @@ int volume_impl(tdm_ctx* c, int n, const VolumeOut& out, cudaStream_t st, CapRec
     float* im = out.im;
     uint8_t* otf = out.otf;
     uint32_t* cnt = out.cnt;
-    using P = PassCfg<D>;
+    using P = ColPass<D>;
     Buffers& b = c->b;
     const Params& p = c->p;
-    const size_t sm_a = GatherZ<D>::smem(p.band, n);
-    const size_t sm_p = P::SMEM;
-    if (sm_a > kMaxSmemPerCta) return TDM_EUNSUPPORTED;
-    if (allow_smem(k_gather_z<D>, sm_a) || allow_smem(k_ypass<D, 1>, sm_p) || allow_smem(k_xpass<D>, sm_p))
-        return TDM_ECUDA;
+    if (allow_smem(k_zpass<D>, P::SMEM)) return TDM_ECUDA;
     // A staged output part may still be downloading from the previous volume:
     // each part's writer waits for that part's download (ev_dl) just before it runs.
     auto staged_free = [&](int part) { return cudaStreamWaitEvent(st, c->ev_dl[part], 0); };
     auto downloaded = [&](int part) { return cudaEventRecord(c->ev_dl[part], c->dl_stream); };
     if (out.host_cnt && staged_free(kOutSlabs)) return TDM_ECUDA;
     if (out.host_otf && staged_free(kOutSlabs + 1)) return TDM_ECUDA;
-    // planes outside the cap band carry no hits and no OTF support
-    const size_t plane = (size_t)D * D, lo = (size_t)p.zmin * plane, hi = (size_t)(p.zmin + p.band) * plane;
-    const size_t NT = (size_t)D * D * D;
+    // cells outside the cap band and outside the columns that caps reach carry no hits and no OTF support
+    const size_t plane = (size_t)D * D, NT = (size_t)D * D * D;
+    const bool all = p.xa == 0 && p.xb == D && p.ya == 0 && p.yb == D;
+    const size_t lo = all ? (size_t)p.zmin * plane : NT, hi = (size_t)(p.zmin + p.band) * plane;
     if (cnt) {
         cudaMemsetAsync(cnt, 0, lo * sizeof(uint32_t), st);
-        cudaMemsetAsync(cnt + hi, 0, (NT - hi) * sizeof(uint32_t), st);
+        if (all) cudaMemsetAsync(cnt + hi, 0, (NT - hi) * sizeof(uint32_t), st);
     }
     if (otf) {
         cudaMemsetAsync(otf, 0, lo, st);
-        cudaMemsetAsync(otf + hi, 0, NT - hi, st);
+        if (all) cudaMemsetAsync(otf + hi, 0, NT - hi, st);
     }
     cudaEventRecord(c->ev_stage[4], st);
-    {
-        Launch l(c, K_GATHER, st);
-        k_gather_z<D><<<dim3(D / 32, D), kGZ * 32, sm_a, st>>>(rec.val, rec.z, posspec, n, p, b.tw, b.vol, cnt, otf,
-                                                                 1);
-    }
+    if (int rc = launch_gather(c, rec, posspec, n, cnt, otf, 1, st)) return rc;
     cudaEventRecord(c->ev_stage[5], st);
     if (ev_gathered && cudaEventRecord(ev_gathered, st)) return TDM_ECUDA;
     if (out.host_cnt) {
@@ -832,29 +851,26 @@ int volume_impl(tdm_ctx* c, int n, const VolumeOut& out, cudaStream_t st, CapRec
         if (download_after(c, st, c->ev_out[kOutSlabs + 1], out.host_otf, otf, NT) || downloaded(kOutSlabs + 1))
             return TDM_ECUDA;
     }
-    {
-        Launch l(c, K_YPASS, st);
-        k_ypass<D, 1><<<dim3(D / P::B, D), P::NT, sm_p, st>>>(b.vol, b.tw);
-    }
-    // x pass by slabs of z blocks; a slab's planes are final once it has run
+    if (int rc = launch_xy<D>(c, st)) return rc;
+    // z pass by slabs of rows y; a slab's rows are final in every plane once it has run
     const bool host_vol = out.host_re || out.host_im;
-    const int zblocks = D / P::B, nslab = host_vol ? (zblocks < kOutSlabs ? zblocks : kOutSlabs) : 1;
+    const int nslab = host_vol ? kOutSlabs : 1;
     for (int sl = 0; sl < nslab; ++sl) {
-        const int zb0 = sl * zblocks / nslab, zb1 = (sl + 1) * zblocks / nslab;
+        const int y0 = sl * D / nslab, y1 = (sl + 1) * D / nslab;
         if (host_vol && staged_free(sl)) return TDM_ECUDA;
         {
-            Launch l(c, K_XPASS, st);
-            k_xpass<D><<<dim3(zb1 - zb0, D), P::NT, sm_p, st>>>(b.vol, b.tw, p.out_scale, zb0, re, im);
+            Launch l(c, K_ZPASS, st);
+            k_zpass<D><<<dim3(D / P::B, y1 - y0), P::NT, P::SMEM, st>>>(b.vol, b.tw, p, p.out_scale, y0, re, im);
         }
         if (host_vol) {
-            const size_t off = (size_t)zb0 * P::B * D * D, len = (size_t)(zb1 - zb0) * P::B * D * D;
+            const size_t off = (size_t)y0 * D, pitch = plane * sizeof(float), width = (size_t)(y1 - y0) * D * sizeof(float);
             if (cudaEventRecord(c->ev_out[sl], st) || cudaStreamWaitEvent(c->dl_stream, c->ev_out[sl], 0))
                 return TDM_ECUDA;
-            if (out.host_re && cudaMemcpyAsync(out.host_re + off, re + off, len * sizeof(float),
-                                               cudaMemcpyDeviceToHost, c->dl_stream))
+            if (out.host_re && cudaMemcpy2DAsync(out.host_re + off, pitch, re + off, pitch, width, D,
+                                                 cudaMemcpyDeviceToHost, c->dl_stream))
                 return TDM_ECUDA;
-            if (out.host_im && cudaMemcpyAsync(out.host_im + off, im + off, len * sizeof(float),
-                                               cudaMemcpyDeviceToHost, c->dl_stream))
+            if (out.host_im && cudaMemcpy2DAsync(out.host_im + off, pitch, im + off, pitch, width, D,
+                                                 cudaMemcpyDeviceToHost, c->dl_stream))
                 return TDM_ECUDA;
             if (downloaded(sl)) return TDM_ECUDA;
         }
@@ -866,24 +882,24 @@ int volume_impl(tdm_ctx* c, int n, const VolumeOut& out, cudaStream_t st, CapRec
 template <int D>
 int forward_impl(tdm_ctx* c, const float* xn, const float* xk, int n, float2* caps, const float2* data, CapRecs res,
                  double* misfit) {
-    using P = PassCfg<D>;
+    using P = ColPass<D>;
+    using R = RowPass<D>;
     Buffers& b = c->b;
     const Params& p = c->p;
-    const size_t sm_p = P::SMEM;
-    if (allow_smem(k_fxpass<D>, sm_p) || allow_smem(k_ypass<D, -1>, sm_p) || allow_smem(k_fzpass<D>, sm_p))
+    if (allow_smem(k_fzpass<D>, P::SMEM) || allow_smem(k_ypass<D, -1>, P::SMEM) || allow_smem(k_xpass<D, -1>, R::SMEM))
         return TDM_ECUDA;
     const float scale = (float)(1.0 / ((double)p.out_scale * (double)D * D * D));
     {
-        Launch l(c, K_XPASS);
-        k_fxpass<D><<<dim3(D / P::B, D), P::NT, sm_p, c->stream>>>(xn, xk, b.tw, scale, b.vol);
+        Launch l(c, K_ZPASS);
+        k_fzpass<D><<<dim3(D / P::B, D), P::NT, P::SMEM, c->stream>>>(xn, xk, b.tw, p, scale, b.vol);
     }
     {
         Launch l(c, K_YPASS);
-        k_ypass<D, -1><<<dim3(D / P::B, D), P::NT, sm_p, c->stream>>>(b.vol, b.tw);
+        k_ypass<D, -1><<<dim3(D / P::B, p.band), P::NT, P::SMEM, c->stream>>>(b.vol, b.tw, p);
     }
     {
-        Launch l(c, K_ZPASS);
-        k_fzpass<D><<<dim3(D * D / P::B), P::NT, sm_p, c->stream>>>(b.vol, b.tw, p.zmin, p.band);
+        Launch l(c, K_XPASS);
+        k_xpass<D, -1><<<(p.band * (p.yb - p.ya) + R::B - 1) / R::B, R::NT, R::SMEM, c->stream>>>(b.vol, b.tw, p);
     }
     {
         Launch l(c, K_CAP_COLS);
@@ -896,45 +912,35 @@ int forward_impl(tdm_ctx* c, const float* xn, const float* xk, int n, float2* ca
 
 template <int D>
 int adjoint_impl(tdm_ctx* c, CapRecs recs, int n, float* xn, float* xk, bool normalize) {
-    using P = PassCfg<D>;
+    using P = ColPass<D>;
     Buffers& b = c->b;
     const Params& p = c->p;
-    const size_t sm_a = GatherZ<D>::smem(p.band, n);
-    const size_t sm_p = P::SMEM;
-    if (sm_a > kMaxSmemPerCta) return TDM_EUNSUPPORTED;
-    if (allow_smem(k_gather_z<D>, sm_a) || allow_smem(k_ypass<D, 1>, sm_p) || allow_smem(k_xpass<D>, sm_p))
-        return TDM_ECUDA;
-    {
-        Launch l(c, K_GATHER);
-        k_gather_z<D><<<dim3(D / 32, D), kGZ * 32, sm_a, c->stream>>>(recs.val, recs.z, b.posspec, n, p, b.tw, b.vol,
-                                                                        nullptr, nullptr, normalize ? 1 : 0);
-    }
-    {
-        Launch l(c, K_YPASS);
-        k_ypass<D, 1><<<dim3(D / P::B, D), P::NT, sm_p, c->stream>>>(b.vol, b.tw);
-    }
+    if (allow_smem(k_zpass<D>, P::SMEM)) return TDM_ECUDA;
+    if (int rc = launch_gather(c, recs, b.posspec, n, nullptr, nullptr, normalize ? 1 : 0, c->stream)) return rc;
+    if (int rc = launch_xy<D>(c, c->stream)) return rc;
     const float scale = normalize ? p.out_scale : (float)(1.0 / ((double)p.out_scale * (double)D * D * D));
     {
-        Launch l(c, K_XPASS);
-        k_xpass<D><<<dim3(D / P::B, D), P::NT, sm_p, c->stream>>>(b.vol, b.tw, scale, 0, xn, xk);
+        Launch l(c, K_ZPASS);
+        k_zpass<D><<<dim3(D / P::B, D), P::NT, P::SMEM, c->stream>>>(b.vol, b.tw, p, scale, 0, xn, xk);
     }
     return cudaGetLastError() == cudaSuccess ? TDM_OK : TDM_ECUDA;
 }
 
 }  // namespace
 
-// Dynamic shared memory of k_gather_z: per warp the sums and counts of its
-// column group (or their exchange buffers), its plane owners and a 32-lane
-// staging row; the CTA's OTF bits and its list of n angles at most.
-size_t gather_smem_bytes(int D, int band, int n) {
-    switch (D) {
-        case 128: return GatherZ<128>::smem(band, n);
-        case 256: return GatherZ<256>::smem(band, n);
-        case 512: return GatherZ<512>::smem(band, n);
-        default: return GatherZ<1024>::smem(band, n);
-    }
+// The angle limit of a context: an angle count is accepted while a list of
+// 8-byte entries fits a CTA's shared memory beside the FP64 sums and counts of
+// four warps' columns (two columns a warp up to D = 512, whose FFT takes half a
+// warp), or their FFT exchange buffers, the plane owners, a staging row and
+// the mask bits.  k_gather, with 4-byte entries, needs less for every band
+// (at most sqrt(2) F + 2 planes, F <= 512) and count that this accepts.
+size_t gather_limit_bytes(int D, int band, int n) {
+    const int T = D / warp_fft_e(D), G = 32 / T;
+    const size_t sums = (size_t)G * band * (sizeof(double2) + sizeof(uint16_t)), xch = (size_t)G * T * (T + 1) * sizeof(float2);
+    const size_t region = ((sums > xch ? sums : xch) + 15) & ~size_t(15);
+    return 4 * (region + 32 * sizeof(float2) + ((band + 15) & ~15)) + (((size_t)band * 4 + 7) & ~size_t(7)) +
+           (size_t)n * sizeof(int2);
 }
-
 int launch_cap(tdm_ctx* c, int a0, int n, bool form) {
     if (c->p.F & (c->p.F - 1)) return launch_cap_generic(c, a0, n, form);
     switch (c->p.F) {

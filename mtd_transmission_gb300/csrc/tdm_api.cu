@@ -300,10 +300,13 @@ int tdm_create(const tdm_geom* geom, int max_angles, tdm_ctx** out) {
         fprintf(stderr, "tdm_create: Ewald caps exceed the DIM_FINAL volume along z\n");
         return TDM_EUNSUPPORTED;
     }
-    if (gather_smem_bytes(D, p.band, max_angles) > kMaxSmemPerCta) {
+    // a cap window's bins lie within F of the centre column; whole 16-column blocks
+    p.xa = p.ya = (D / 2 - F) & ~15;
+    p.xb = p.yb = (D / 2 + F + 15) & ~15;
+    if (gather_limit_bytes(D, p.band, max_angles) > kMaxSmemPerCta) {
         // the gather keeps each CTA's list of angles in shared memory
         int most = 0;
-        while (gather_smem_bytes(D, p.band, most + 1) <= kMaxSmemPerCta) ++most;
+        while (gather_limit_bytes(D, p.band, most + 1) <= kMaxSmemPerCta) ++most;
         delete c;
         fprintf(stderr, "tdm_create: at most %d angles for this geometry (the cap gather's angle list of a "
                         "%d-plane cap band must fit one CTA's shared memory)\n", most, p.band);
@@ -393,7 +396,7 @@ int tdm_create(const tdm_geom* geom, int max_angles, tdm_ctx** out) {
     TRY(dev_alloc(c, &b.posspec_vol[0], M));
     TRY(dev_alloc(c, &b.posspec_vol[1], M));
     b.rec = b.rec_buf[0];
-    TRY(dev_alloc(c, &b.vol, (size_t)D * D * D));
+    TRY(dev_alloc(c, &b.vol, (size_t)p.band * D * D));
     TRY(dev_alloc(c, &b.rinv, kNC * kNC));
     TRY(dev_alloc(c, &b.err, 4));
     // tables

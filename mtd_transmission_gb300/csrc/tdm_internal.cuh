@@ -13,7 +13,7 @@
 namespace tdm {
 
 constexpr int kNC = 15;  // degree-4 2D polynomial: 15 monomials
-constexpr int kOutSlabs = 8;  // x-pass slabs whose outputs are downloaded while the next slab runs
+constexpr int kOutSlabs = 4;  // z-pass slabs (rows y) whose outputs are downloaded while the next slab runs
 constexpr int kOutEvents = kOutSlabs + 2;
 constexpr int kMaxLanes = 8;    // chunks of the per-angle stages in flight at once
 constexpr int kStageSlots = 16; // hologram upload slots of one chunk each
@@ -35,6 +35,7 @@ struct Params {
     int volkov;              // VOLKOV: 1 Volkov unwrapping, 0 Herraez
     int disc_thr;            // fd^2 < disc_thr  <=>  fd^2 < COEF_NA_OBJ_LIMIT * N^2
     int zmin, band;          // cap planes z in [zmin, zmin + band)
+    int xa, xb, ya, yb;      // voxel columns that caps reach: X in [xa, xb), Y in [ya, yb), multiples of 16
     int r2i;                 // rayon^2 when below 2^24 (cap heights as float sqrt of exact integers), else 0
     double rayon, inv_rayon;
     float cap_scale;         // (k0/pi)*(-2pi) of retroPropag_Born, k0 in float
@@ -81,7 +82,7 @@ struct Buffers {
     CapRecs rec;                   // max_angles x F*F cap records: rec_buf[i]
     CapRecs rec_buf[2];            // the two cap-record buffers of consecutive pipeline calls
     int2* posspec_vol[2] = {};     // max_angles: specular positions read by the volume stage of those calls
-    float2* vol = nullptr;         // D^3 complex, [y][x][z] layout
+    float2* vol = nullptr;         // band x D^2 complex: the spectrum's cap planes, [z - zmin][y][x]
     float* out_re = nullptr;       // D^3 staging when the caller's output is in host memory
     float* out_im = nullptr;
     uint8_t* out_otf = nullptr;
@@ -133,7 +134,7 @@ struct tdm_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;  // hologram uploads
     cudaStream_t dl_stream = nullptr;    // output downloads (a second copy engine)
-    // downloads of the staged outputs done, per part (x-pass slabs, then counts, then OTF): a volume
+    // downloads of the staged outputs done, per part (z-pass slabs, then counts, then OTF): a volume
     // stage waits for the previous volume's download of a part just before it rewrites that part
     cudaEvent_t ev_dl[tdm::kOutEvents] = {};
     // tdm_pipeline runs each volume's stage (gather, z/y/x passes) on vol_stream, so that it
@@ -163,9 +164,9 @@ struct tdm_ctx {
 
 // Kernel launchers (defined in the kernel translation units).
 namespace tdm {
-// Dynamic shared memory of the cap gather for a cap band of `band` planes and
-// n angles (the CTA keeps its list of angles in shared memory).
-size_t gather_smem_bytes(int D, int band, int n);
+// Shared memory that sets a context's angle limit, for a cap band of `band`
+// planes and n angles (the gather keeps each CTA's list of angles there).
+size_t gather_limit_bytes(int D, int band, int n);
 constexpr size_t kMaxSmemPerCta = 227 * 1024;
 // Scope around one kernel launch on c->stream: counts the launch and, when
 // profiling is on, brackets it with a pair of CUDA events.
@@ -232,7 +233,7 @@ void launch_form(tdm_ctx* c, const float* unw, int g0, int m);
 // Outputs of the volume stage: the device buffers the kernels write and, for
 // each caller buffer in host memory, the host destination its device copy is
 // downloaded to on the copy stream as soon as the pass that completes it has
-// run (the index and absorption volumes slab by slab during the x pass).
+// run (the index and absorption volumes slab by slab during the z pass).
 struct VolumeOut {
     float* re = nullptr;
     float* im = nullptr;
@@ -250,7 +251,7 @@ struct VolumeOut {
 int launch_forward(tdm_ctx* c, const float* xn, const float* xk, int n, float2* caps, const float2* data,
                    CapRecs res, double* misfit);
 // Adjoint of the forward operator applied to cap records (unnormalised
-// scatter, z/y/x passes); with normalize, the hit-count-normalised scatter and
+// scatter, x/y/z passes); with normalize, the hit-count-normalised scatter and
 // the reconstruction's own scale (the single-pass reconstruction of recs).
 int launch_adjoint(tdm_ctx* c, CapRecs recs, int n, float* xn, float* xk, bool normalize);
 // Cap records (value, cell plane) of cap values in FFT-bin order.
@@ -261,7 +262,7 @@ int launch_tv_step(tdm_ctx* c, const float* xn, const float* xk, const float* gn
                    float* xk_out);
 // gather of the cap records rec (angles [0, n), specular positions posspec),
 // normalisation and 3D inverse FFT into the outputs, on stream st.  Downloads
-// run on c->dl_stream; each staged part (x-pass slab, counts, OTF) is
+// run on c->dl_stream; each staged part (z-pass slab, counts, OTF) is
 // rewritten only after the previous volume's download of that part is done
 // (c->ev_dl).  ev_gathered (may be null) is recorded on st once the gather
 // has read rec.
