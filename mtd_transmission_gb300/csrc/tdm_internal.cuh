@@ -209,7 +209,6 @@ int launch_extract(tdm_ctx* c, const void* holos_dev, int bits, int n, int a0, b
 // Herraez unwrapping (VOLKOV 0) of the chunk's m wrapped phases (b.phase ->
 // b.unwrapped), stack angles a0 .. a0 + m - 1; F <= 256.
 int launch_herraez(tdm_ctx* c, int a0, int m);
-size_t herraez_gather_smem(int F);
 int launch_fields(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapped, float* dbg_amp,
                   int argparts = 0, bool form = true);
 // Per-field spectra and cap contributions for fields [a0, a0 + n); with
