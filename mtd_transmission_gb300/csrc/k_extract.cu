@@ -34,8 +34,9 @@ int extract_impl(tdm_ctx* c, const void* holos, int bits, int n, int a0, bool ar
     const bool bulk = (reinterpret_cast<uintptr_t>(holos) & 15) == 0;
     auto rows = bulk ? k_extract_rows<H, true> : k_extract_rows<H, false>;
     const size_t bytes_per = (size_t)H * H * (bits == 16 ? 2 : 1);
-    for (int h0 = 0; h0 < n; h0 += c->holo_chunk) {
-        const int m = n - h0 < c->holo_chunk ? n - h0 : c->holo_chunk;
+    const int step = angles_per_launch(c, n);
+    for (int h0 = 0; h0 < n; h0 += step) {
+        const int m = n - h0 < step ? n - h0 : step;
         const char* src = static_cast<const char*>(holos) + (size_t)h0 * bytes_per;
         {
             Launch l(c, K_EXTRACT_ROWS);

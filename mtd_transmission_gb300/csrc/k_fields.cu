@@ -655,8 +655,9 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
         allow_smem(k_volkov_rows<L>, sm_vrows) || allow_smem(k_volkov_cols<L>, sm_vcols) ||
         allow_smem(k_volkov_integ_rows<F>, IC::SMEM) || allow_smem(k_volkov_integ_cols<F>, IC::SMEM))
         return TDM_ECUDA;
-    for (int g0 = a0; g0 < a0 + n; g0 += c->chunk) {
-        const int m = (a0 + n - g0) < c->chunk ? (a0 + n - g0) : c->chunk;
+    const int step = angles_per_launch(c, n);
+    for (int g0 = a0; g0 < a0 + n; g0 += step) {
+        const int m = a0 + n - g0 < step ? a0 + n - g0 : step;
         const float2* spec = b.spectra + (size_t)g0 * FF;
         int nparts = argparts;
         if (!nparts) {

@@ -469,8 +469,9 @@ int gfields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapp
         allow_smem(gk_volkov_integ_rows<F>, sm_irows) || allow_smem(gk_volkov_integ_cols<F>, sm_icols))
         return TDM_ECUDA;
     const unsigned rows = (F + kRows - 1) / kRows, cols = (F + kCols - 1) / kCols;
-    for (int g0 = a0; g0 < a0 + n; g0 += c->chunk) {
-        const int m = (a0 + n - g0) < c->chunk ? (a0 + n - g0) : c->chunk;
+    const int step = angles_per_launch(c, n);
+    for (int g0 = a0; g0 < a0 + n; g0 += step) {
+        const int m = a0 + n - g0 < step ? a0 + n - g0 : step;
         const float2* spec = b.spectra + (size_t)g0 * FF;
         const int nparts = argparts ? argparts : launch_argmax_part(c, spec, m);
         {
@@ -533,8 +534,9 @@ int gcap_impl(tdm_ctx* c, int a0, int n, bool form) {
     if (form && n > c->chunk) return TDM_EINVAL;  // the chunk buffers hold one chunk
     const size_t FF = (size_t)F * F;
     const unsigned rows = (F + kRows - 1) / kRows, cols = (F + kCols - 1) / kCols;
-    for (int g0 = a0; g0 < a0 + n; g0 += c->chunk) {
-        const int m = a0 + n - g0 < c->chunk ? a0 + n - g0 : c->chunk;
+    const int step = angles_per_launch(c, n);
+    for (int g0 = a0; g0 < a0 + n; g0 += step) {
+        const int m = a0 + n - g0 < step ? a0 + n - g0 : step;
         {
             Launch l(c, K_CAP_ROWS);
             if (form)

@@ -747,8 +747,9 @@ int cap_impl(tdm_ctx* c, int a0, int n, bool form) {
         return TDM_ECUDA;
     if (form && n > c->chunk) return TDM_EINVAL;  // the chunk buffers hold one chunk
     const size_t FF = (size_t)F * F;
-    for (int g0 = a0; g0 < a0 + n; g0 += c->chunk) {
-        const int m = a0 + n - g0 < c->chunk ? a0 + n - g0 : c->chunk;
+    const int step = angles_per_launch(c, n);
+    for (int g0 = a0; g0 < a0 + n; g0 += step) {
+        const int m = a0 + n - g0 < step ? a0 + n - g0 : step;
         if (form) {
             Launch l(c, K_CAP_ROWS);
             k_cap_rows_form<F><<<dim3(F / C::B, m), C::NT, C::SMEM, c->stream>>>(

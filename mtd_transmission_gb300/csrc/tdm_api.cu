@@ -259,6 +259,12 @@ int tdm_create(const tdm_geom* geom, int max_angles, tdm_ctx** out) {
     p.rayon = c->dv.rayon;
     p.inv_rayon = 1.0 / c->dv.rayon;
     const int N = p.N, F = p.F, D = p.D;
+    // The pipeline's chunks: a quarter of the scratch each (200 x 512^2: (32, 4) 0.48, (16, 4) 0.65 ms a volume; 400
+    // x 256^2: 0.40, 0.64), but no more angles in flight than leave the extraction's band, the largest hand-over
+    // between two kernels, in L2 (600 x 1024^2, three contexts at once: (16, 4) 4.29, (32, 4) 4.42 ms), and no
+    // chunks of a few angles, whose launches cost more than they fill.
+    const int fit = (int)(kL2Bytes / ((size_t)p.H * F * sizeof(float2)));
+    c->chunk = c->holo_chunk = std::max(16, std::min(c->chunk_cap, fit) / c->lanes);
     // disc test fd^2 < COEF_NA_OBJ_LIMIT * N^2 on integers (fonctions.cpp:915)
     const double lim = geom->coef_na_obj_limit * (double)(N * N);
     p.disc_thr = (int)std::min<double>(std::ceil(lim), 2.0 * N * N + 1);
@@ -422,8 +428,6 @@ int tdm_create(const tdm_geom* geom, int max_angles, tdm_ctx** out) {
         cudaMemset(b.fit_done, 0, CH * 2 * sizeof(unsigned)) != cudaSuccess)
         TRY(cuda_fail(c, cudaGetLastError(), "table upload"));
     if (p.c_aber && p.deroul && !p.volkov) {  // Herraez unwrapping's border reliabilities
-        // its merging runs one CTA per angle: twice as many angles in flight
-        if (32 * c->lanes <= c->chunk_cap) c->chunk = c->holo_chunk = 32;
         const std::vector<int> br = crand_border_table(F, max_angles);
         TRY(dev_alloc(c, &b.hz_rand, br.size()));
         if (cudaMemcpy(b.hz_rand, br.data(), br.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)

@@ -17,6 +17,7 @@ constexpr int kOutSlabs = 4;  // z-pass slabs (rows y) whose outputs are downloa
 constexpr int kOutEvents = kOutSlabs + 2;
 constexpr int kMaxLanes = 8;    // chunks of the per-angle stages in flight at once
 constexpr int kStageSlots = 16; // hologram upload slots of one chunk each
+constexpr size_t kL2Bytes = size_t(126) << 20;
 constexpr int kChunkCapMax = 128;  // angles of per-chunk scratch (all lanes together), at most
 
 // Cap records of a stack: per angle and FFT bin ([angle][ky][kx]) the cap
@@ -119,7 +120,7 @@ struct tdm_ctx {
     tdm::Params p{};
     tdm::Buffers b{};
     int max_angles = 0;
-    int chunk = 16;              // angles per chunk of the per-angle stages (tdm_set_schedule, tdm_autotune)
+    int chunk = 16;              // angles per chunk of the pipeline's per-angle stages (tdm_set_schedule, tdm_autotune)
     int holo_chunk = 16;         // holograms per extraction chunk (equal to chunk)
     int lanes = 4;               // chunks in flight at once; lanes * chunk <= chunk_cap
     int chunk_cap = 64;          // angles of per-chunk scratch: min(128, max_angles rounded up to 16)
@@ -198,6 +199,17 @@ struct Launch {
 // must not lower it under a launch (or a captured graph) that needs more.
 cudaError_t max_dynamic_smem(const void* fn, size_t bytes);
 
+// Angles per launch for n angles through the whole scratch, in equal parts:
+// the entry points of the single stages run their launches one after the
+// other, and one as large as the scratch allows fills the GPU where one of 16
+// angles leaves most of it idle (200 fields of 256^2: 16 angles 1187 us, 32 909,
+// 64 759, 128 681; extraction of 400 x 1024^2: 1080, 952, 899, 840, although its
+// 2 MB an angle between the passes no longer stay in L2).  The pipeline passes
+// at most one chunk, which is one part.
+inline int angles_per_launch(const tdm_ctx* c, int n) {
+    const int parts = (n + c->chunk_cap - 1) / c->chunk_cap;
+    return (n + parts - 1) / parts;
+}
 // Extraction of holograms [0, n) from device memory into spectra[a0, a0 + n).
 // With argmax = true (n at most one chunk), the column pass also leaves the
 // specular search's partial winners of each angle in b.argpart; the return
