@@ -38,12 +38,25 @@ __host__ __device__ constexpr int padded_len(int n) { return n + (n >> 4); }
 __host__ __device__ constexpr int tstride(int n) { return padded_len(n) + 1; }
 __host__ __device__ constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c(n >> 1); }
 
-__device__ __forceinline__ float2 c_add(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 c_sub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// A complex value is a register pair, and the packed FP32 instructions of this
+// GPU work on both halves at once: an addition, a real scaling or a butterfly
+// with a common real factor is one instruction instead of two.  (A product
+// with a complex factor or +-i would need the halves swapped by moves first, so
+// those stay scalar.)  The FFT passes issue two thirds of their instructions
+// for arithmetic: extraction of 400 x 1024^2 row pass 512 -> 478 us, column pass
+// 280 -> 262 us, a 600 x 1024^2 volume 4.02 -> 3.90 ms.
+__device__ __forceinline__ float2 c_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 c_sub(float2 a, float2 b) {
+    float2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long&>(r))
+        : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
+    return r;
+}
 __device__ __forceinline__ float2 c_mul(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
 }
-__device__ __forceinline__ float2 c_scale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
+__device__ __forceinline__ float2 c_scale(float2 a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
 __device__ __forceinline__ float2 c_conj(float2 a) { return make_float2(a.x, -a.y); }
 
 // a * (DIR * i)
@@ -61,12 +74,12 @@ __device__ __forceinline__ void dft2(float2& a0, float2& a1) {
 
 template <int DIR>
 __device__ __forceinline__ void dft4(float2& a0, float2& a1, float2& a2, float2& a3) {
-    float2 t0 = c_add(a0, a2), t1 = c_sub(a0, a2);
-    float2 t2 = c_add(a1, a3), t3 = mul_dir_i<DIR>(c_sub(a1, a3));
+    const float2 t0 = c_add(a0, a2), t1 = c_sub(a0, a2);
+    const float2 t2 = c_add(a1, a3), d = c_sub(a1, a3);
     a0 = c_add(t0, t2);
     a2 = c_sub(t0, t2);
-    a1 = c_add(t1, t3);
-    a3 = c_sub(t1, t3);
+    a1 = make_float2(t1.x - DIR * d.y, t1.y + DIR * d.x);  // t1 + DIR i d
+    a3 = make_float2(t1.x + DIR * d.y, t1.y - DIR * d.x);
 }
 
 template <int DIR>
@@ -76,18 +89,18 @@ __device__ __forceinline__ void dft8(float2* x) {
     dft4<DIR>(e0, e1, e2, e3);
     dft4<DIR>(o0, o1, o2, o3);
     const float r = 0.70710678118654752440f;
-    // o1 *= exp(DIR i pi/4), o2 *= DIR i, o3 *= exp(DIR 3 i pi/4)
-    o1 = make_float2(r * (o1.x - DIR * o1.y), r * (DIR * o1.x + o1.y));
-    o2 = mul_dir_i<DIR>(o2);
-    o3 = make_float2(-r * (o3.x + DIR * o3.y), r * (DIR * o3.x - o3.y));
+    const float2 rp = make_float2(r, r), rm = make_float2(-r, -r);
+    // o1 *= exp(DIR i pi/4) = r u1, o2 *= DIR i, o3 *= exp(DIR 3 i pi/4) = r u3
+    const float2 u1 = make_float2(o1.x - DIR * o1.y, DIR * o1.x + o1.y);
+    const float2 u3 = make_float2(-o3.x - DIR * o3.y, DIR * o3.x - o3.y);
     x[0] = c_add(e0, o0);
     x[4] = c_sub(e0, o0);
-    x[1] = c_add(e1, o1);
-    x[5] = c_sub(e1, o1);
-    x[2] = c_add(e2, o2);
-    x[6] = c_sub(e2, o2);
-    x[3] = c_add(e3, o3);
-    x[7] = c_sub(e3, o3);
+    x[1] = __ffma2_rn(rp, u1, e1);
+    x[5] = __ffma2_rn(rm, u1, e1);
+    x[2] = make_float2(e2.x - DIR * o2.y, e2.y + DIR * o2.x);
+    x[6] = make_float2(e2.x + DIR * o2.y, e2.y - DIR * o2.x);
+    x[3] = __ffma2_rn(rp, u3, e3);
+    x[7] = __ffma2_rn(rm, u3, e3);
 }
 
 // One Stockham stage on a transform held in shared memory (in place).
