@@ -224,17 +224,40 @@ __device__ __forceinline__ void fft_warp_regs(float2 (&x)[WarpFFT<N>::E], float2
     for (int q = 0; q < E / T; ++q) dft<T, DIR>(&x[q * T]);
 }
 
-// fft_warp_regs for a transform whose T lanes sit in several warps of the CTA
-// (a pass whose lanes run across transforms, so that it loads and stores
-// columns directly): the exchange is ordered by CTA barriers.  s must not be
-// in use on entry; every thread of the CTA calls it together, once.
-template <int N, int DIR>
+// Column passes: a CTA transforms B neighbouring columns of a row-major array
+// and its lanes run across them, so that loads and stores go straight between
+// registers and global memory in whole lines, and shared memory holds the
+// transforms' exchanges only, ordered by CTA barriers (a warp per transform
+// needs the columns staged and unstaged through shared memory, which is three
+// times the traffic there).  A warp holds B = 16 columns of two lanes j: lane
+// pairs j and T - j (0 and T/2 in warp 0), so that bin N - k is held 16 lanes
+// away (in warp 0 by the lane itself), as the mirror passes want it.
+template <int N>
+struct ColFFT {
+    using W = WarpFFT<N>;
+    static constexpr int B = 16;
+    static constexpr int NT = B * W::T;
+    static constexpr size_t SMEM = (size_t)B * W::STRIDE * sizeof(float2);
+    __device__ static int column() { return threadIdx.x % B; }
+    __device__ static int adjacent_j() { return threadIdx.x / B; }
+    __device__ static int paired_j() {
+        const int w = threadIdx.x >> 5;
+        return (threadIdx.x & 16) ? (w ? W::T - w : W::T / 2) : w;
+    }
+    __device__ static int partner() { return threadIdx.x < 32 ? threadIdx.x & 31 : (threadIdx.x & 31) ^ 16; }
+};
+
+// fft_warp_regs and fft_warp_regs_rev for such a pass (s: the column's array).
+// FIRST: nothing in s is still to be read by other threads on entry.
+// Every thread of the CTA calls them together.
+template <int N, int DIR, bool FIRST = true>
 __device__ __forceinline__ void fft_cta_regs(float2 (&x)[WarpFFT<N>::E], float2* s, int j,
                                              const float2* __restrict__ tw) {
     using W = WarpFFT<N>;
     constexpr int E = W::E, T = W::T;
     dft<E, DIR>(x);
     twiddle_lane<N, DIR>(x, tw + twr_offset(N), j);
+    if (!FIRST) __syncthreads();
 #pragma unroll
     for (int k1 = 0; k1 < E; ++k1) s[k1 * (T + 1) + j] = x[k1];  // pad(k1 T + j)
     __syncthreads();
@@ -245,6 +268,26 @@ __device__ __forceinline__ void fft_cta_regs(float2 (&x)[WarpFFT<N>::E], float2*
     }
 #pragma unroll
     for (int q = 0; q < E / T; ++q) dft<T, DIR>(&x[q * T]);
+}
+
+template <int N, int DIR, bool FIRST = true>
+__device__ __forceinline__ void fft_cta_regs_rev(float2 (&x)[WarpFFT<N>::E], float2* s, int j,
+                                                 const float2* __restrict__ tw) {
+    using W = WarpFFT<N>;
+    constexpr int E = W::E, T = W::T;
+#pragma unroll
+    for (int q = 0; q < E / T; ++q) dft<T, DIR>(&x[q * T]);
+    if (!FIRST) __syncthreads();
+#pragma unroll
+    for (int q = 0; q < E / T; ++q) {
+#pragma unroll
+        for (int n2 = 0; n2 < T; ++n2) s[(j + q * T) * (T + 1) + n2] = x[q * T + n2];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k1 = 0; k1 < E; ++k1) x[k1] = s[k1 * (T + 1) + j];
+    twiddle_lane<N, DIR>(x, tw + twr_offset(N), j);
+    dft<E, DIR>(x);
 }
 
 // The same transform run from the other end: on entry x[q T + k2] holds

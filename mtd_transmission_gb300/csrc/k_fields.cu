@@ -117,49 +117,48 @@ k_field_rows(const float2* __restrict__ spectra, const float4* __restrict__ argp
     }
 }
 
-// mode 1: phase/amplitude (C_ABER); mode 0: the field itself is the result.
-// mode 1 also leaves the CTA's sum of the wrapped phase in
+// Columns (ColFFT).  mode 1: phase/amplitude (C_ABER); mode 0: the field
+// itself is the result.  mode 1 also leaves the CTA's sum of the wrapped phase in
 // psum[a * kPhaseParts + blockIdx.x] (FP32 per thread and warp, FP64 across
-// the warps in a fixed order).
+// the warps in a fixed order).  phase may be null (Volkov: only the sum is used).
 template <int F>
-__global__ void __launch_bounds__(FieldCfg<F>::NT)
+__global__ void __launch_bounds__(ColFFT<F>::NT)
 k_field_cols(const float2* __restrict__ I1, int mode, const float2* __restrict__ tw, float* __restrict__ phase,
              float* __restrict__ amp, float2* __restrict__ zph, float2* __restrict__ fields,
              double* __restrict__ psum) {
-    using C = FieldCfg<F>;
+    using C = ColFFT<F>;
     using W = typename C::W;
-    constexpr int B = C::B, NT = C::NT;
+    constexpr int T = W::T, E = W::E;
     extern __shared__ float2 sm[];
-    const int tr = threadIdx.x / W::T, j = threadIdx.x % W::T;
-    const int a = blockIdx.y, x0 = blockIdx.x * B;
-#pragma unroll  // every staging load in flight before the first store
-    for (int r0 = 0; r0 < B * F / NT; ++r0) {
-        const int i = threadIdx.x + r0 * NT, t = i % B, r = i / B;
-        sm[t * W::STRIDE + W::pad(r)] = I1[((size_t)a * F + r) * F + x0 + t];
-    }
-    __syncthreads();
-    fft_warp<F, +1>(sm + tr * W::STRIDE, j, tw);
-    __syncthreads();
+    const int t = C::column(), j = C::adjacent_j();
+    const int a = blockIdx.y, xi = blockIdx.x * C::B + t, xo = (xi + F / 2) & (F - 1);
+    const float2* col = I1 + (size_t)a * F * F + xi;
+    float2 x[E];
+#pragma unroll
+    for (int n1 = 0; n1 < E; ++n1) x[n1] = col[(j + n1 * T) * F];
+    fft_cta_regs<F, +1>(x, sm + t * W::STRIDE, j, tw);
     float acc = 0.0f;
-#pragma unroll 8
-    for (int r0 = 0; r0 < B * F / NT; ++r0) {
-        const int i = threadIdx.x + r0 * NT, t = i % B, y = i / B;
-        const float2 u = sm[t * W::STRIDE + W::pad(y)];
-        const int yo = (y + F / 2) & (F - 1), xo = (x0 + t + F / 2) & (F - 1);
-        const size_t o = ((size_t)a * F + yo) * F + xo;
-        if (mode) {
-            const float m = hypotf(u.x, u.y);
-            const float ph = atan2f(u.y, u.x);
-            phase[o] = ph;
-            acc += ph;
-            amp[o] = m;
-            // exp(i phase) without the round trip through the angle; atan2(0, 0) = 0
-            zph[o] = m > 0.0f ? make_float2(u.x / m, u.y / m) : make_float2(1.0f, 0.0f);
-        } else {
-            fields[o] = u;
+#pragma unroll
+    for (int q = 0; q < E / T; ++q) {
+#pragma unroll
+        for (int k2 = 0; k2 < T; ++k2) {
+            const float2 u = x[q * T + k2];
+            const int yo = (j + q * T + E * k2 + F / 2) & (F - 1);
+            const size_t o = ((size_t)a * F + yo) * F + xo;
+            if (mode) {
+                const float m = hypotf(u.x, u.y);
+                const float ph = atan2f(u.y, u.x);
+                if (phase) phase[o] = ph;
+                acc += ph;
+                amp[o] = m;
+                // exp(i phase) without the round trip through the angle; atan2(0, 0) = 0
+                zph[o] = m > 0.0f ? make_float2(u.x / m, u.y / m) : make_float2(1.0f, 0.0f);
+            } else {
+                fields[o] = u;
+            }
         }
     }
-    if (mode) phase_sum_cta<NT>(acc, psum + (size_t)a * kPhaseParts + blockIdx.x);
+    if (mode) phase_sum_cta<C::NT>(acc, psum + (size_t)a * kPhaseParts + blockIdx.x);
 }
 
 // ---------------------------------------------------------------- Volkov unwrap
@@ -178,18 +177,51 @@ k_field_cols(const float2* __restrict__ I1, int mode, const float2* __restrict__
 // kappa(k)/2F, inverse), from two F-point transforms instead of two 2F-point ones.
 __host__ __device__ constexpr int mirror_pos(int m, int F) { return m < F / 2 ? 2 * m : 2 * (F - 1 - m) + 1; }
 
-// x[n1] holds row sample mirror_pos(j + T n1) on entry and the derivative at
-// X = F + mirror_pos(j + T n1) on return; s is the transform's exchange array.
+// The transforms of a pass: s is the transform's exchange array, j the lane in
+// the transform, partner the warp lane that holds bins F - k of its own bins k.
 template <int F>
-__device__ __forceinline__ void mirror_derivative(float2 (&x)[WarpFFT<F>::E], float2* s, int j,
+struct RowLanes {  // a warp per G transforms
+    static constexpr int T = WarpFFT<F>::T;
+    float2* s;
+    int j;
+    __device__ int partner() const { return ((threadIdx.x & 31) & ~(T - 1)) + ((T - j) & (T - 1)); }
+    template <int DIR, bool FIRST>
+    __device__ __forceinline__ void fwd(float2 (&x)[WarpFFT<F>::E], const float2* __restrict__ tw) const {
+        fft_warp_regs<F, DIR>(x, s, j, tw);
+    }
+    template <int DIR>
+    __device__ __forceinline__ void rev(float2 (&x)[WarpFFT<F>::E], const float2* __restrict__ tw) const {
+        fft_warp_regs_rev<F, DIR>(x, s, j, tw);
+    }
+};
+template <int F>
+struct ColLanes {  // lanes across columns (ColFFT)
+    float2* s;
+    int j;
+    __device__ int partner() const { return ColFFT<F>::partner(); }
+    template <int DIR, bool FIRST>
+    __device__ __forceinline__ void fwd(float2 (&x)[WarpFFT<F>::E], const float2* __restrict__ tw) const {
+        fft_cta_regs<F, DIR, FIRST>(x, s, j, tw);
+    }
+    template <int DIR, bool FIRST = false>
+    __device__ __forceinline__ void rev(float2 (&x)[WarpFFT<F>::E], const float2* __restrict__ tw) const {
+        fft_cta_regs_rev<F, DIR, FIRST>(x, s, j, tw);
+    }
+};
+
+// x[n1] holds row sample mirror_pos(j + T n1) on entry and the derivative at
+// X = F + mirror_pos(j + T n1) on return.
+template <int F, class Lanes>
+__device__ __forceinline__ void mirror_derivative(float2 (&x)[WarpFFT<F>::E], const Lanes& ln,
                                                   const float2* __restrict__ tw) {
     using W = WarpFFT<F>;
     constexpr int E = W::E, T = W::T, L = 2 * F;
-    fft_warp_regs<F, -1>(x, s, j, tw);
+    const int j = ln.j;
+    ln.template fwd<-1, true>(x, tw);
     // bin k = (j + qT) + E k2 is in x[qT + k2]; bin F - k is held by lane T - j of
     // the transform, register (E/T - 1 - q)T + (T - 1 - k2), and for lane 0 by
     // itself, register (T - k2) mod T when q = 0, (E/T - q)T + T - 1 - k2 otherwise
-    const int src = ((threadIdx.x & 31) & ~(T - 1)) + ((T - j) & (T - 1));
+    const int src = ln.partner();
     float2 el[E / T];  // e^{i pi (j + qT)/F}
 #pragma unroll
     for (int q = 0; q < E / T; ++q) {
@@ -211,7 +243,7 @@ __device__ __forceinline__ void mirror_derivative(float2 (&x)[WarpFFT<F>::E], fl
             y[q * T + k2] = k == 0 ? make_float2(0.0f, 0.0f) : make_float2(-c * t.y, c * t.x);
         });
     });
-    fft_warp_regs_rev<F, +1>(y, s, j, tw);
+    ln.template rev<+1>(y, tw);
 #pragma unroll
     for (int n1 = 0; n1 < E; ++n1) x[n1] = (j + n1 * T < F / 2) ? y[n1] : make_float2(-y[n1].x, -y[n1].y);
 }
@@ -227,14 +259,14 @@ __device__ __forceinline__ void mirror_derivative(float2 (&x)[WarpFFT<F>::E], fl
 //     DST-II(b)[k] = Re(w V[k] - conj(w) V[F-k]) / 2.
 // x holds a + i (-1)^y b permuted (x[n1] = element j + T n1) on entry;
 // out(k, (DCT-II(a)[k], DST-II(b)[k])) receives every bin k in [0, F) once.
-template <int F, class Out>
-__device__ __forceinline__ void column_dct_dst(float2 (&x)[WarpFFT<F>::E], float2* s, int j,
+template <int F, class Lanes, class Out>
+__device__ __forceinline__ void column_dct_dst(float2 (&x)[WarpFFT<F>::E], const Lanes& ln,
                                                const float2* __restrict__ tw, Out&& out) {
     using W = WarpFFT<F>;
     constexpr int E = W::E, T = W::T, L = 2 * F;
-    fft_warp_regs<F, -1>(x, s, j, tw);
-    __syncwarp();  // the transform is done with s, which out() may overwrite
-    const int src = ((threadIdx.x & 31) & ~(T - 1)) + ((T - j) & (T - 1));  // holder of bin F - k
+    const int j = ln.j;
+    ln.template fwd<-1, false>(x, tw);
+    const int src = ln.partner();  // holder of bin F - k
     float2 wl[E / T];  // e^{-i pi (j + qT)/2F}
 #pragma unroll
     for (int q = 0; q < E / T; ++q) wl[q] = __ldg(&tw[(j + q * T) * (kTwN / (2 * L))]);
@@ -263,25 +295,6 @@ struct RCfg {
     static constexpr size_t SMEM = (size_t)B * W::STRIDE * sizeof(float2);
 };
 
-// Pass 2 in CTAs of NC = 8 mirror columns: NC F-point derivative transforms
-// of Z, then NC F-point transforms giving each column's DCT-II of gx and
-// DST-II of gy (column_dct_dst), staged in its Q array.
-template <int L>
-struct VCfg {
-    using WF = WarpFFT<L / 2>;
-    static constexpr int NC = 8;                 // columns per CTA
-    static constexpr int BF = NC;                // derivative transforms per CTA
-    static_assert(NC % WF::G == 0, "whole warps");
-    static constexpr int NT = BF * WF::T;
-    // array stride 2 mod 16 float2 and at least F: a warp's 8 columns x 4 rows
-    // of the staging loops land in distinct banks
-    static constexpr int FS = WF::LEN + ((2 - WF::LEN % 16) + 16) % 16;
-    static constexpr size_t SMEM_COLS = (size_t)(BF + NC) * FS * sizeof(float2);
-    // CTAs per SM the registers are bounded for (up to L = 512; larger mirrors
-    // need their registers)
-    static constexpr int COLS_CTAS = L <= 512 ? 4 : 1;
-};
-
 // Pass 1: rows of the mirror.  Mirror rows Y and L-1-Y are the same image
 // row, and only the right half of the phasor's gradient
 // gx = Re(-i dZ/dx / Z) / 2pi is kept: gx[Y][X] = sign(X) gxh[m(Y)][m(X)].
@@ -303,7 +316,7 @@ k_volkov_rows(const float2* __restrict__ zph, const float2* __restrict__ tw, flo
     float2 x[E];
 #pragma unroll
     for (int n1 = 0; n1 < E; ++n1) x[n1] = zr[mirror_pos(j + n1 * T, F)];
-    mirror_derivative<F>(x, s, j, tw);
+    mirror_derivative<F>(x, RowLanes<F>{s, j}, tw);
     __syncwarp();  // the transform's exchanges are done with s
 #pragma unroll
     for (int n1 = 0; n1 < E; ++n1) s[W::pad(mirror_pos(j + n1 * T, F))] = x[n1];
@@ -323,67 +336,38 @@ k_volkov_rows(const float2* __restrict__ zph, const float2* __restrict__ tw, flo
 // transforms: along y, gx (even about the mirror's axis) is a DCT-II and gy
 // (odd) a DST-II of the quadrant's column, c[ky][x] = (DCT-II_y gx,
 // DST-II_y gy) for ky in [0, F) (column_dct_dst).  The derivatives come from
-// F-point transforms on the half Y = F + y (mirror_derivative).  The loads and
-// the gy epilogue run CTA-wide with the NC columns fastest (contiguous in
-// global memory); the phasor and gx are read from L2 in the epilogue.
+// F-point transforms on the half Y = F + y (mirror_derivative).  All of it in
+// registers between the loads and the stores (ColFFT): a thread's derivatives
+// are those of the rows it loaded, and gx + i (-1)^y gy of these rows is the
+// next transform's input element.  200 angles of 256^2: 167 us with the columns
+// and the products staged through shared memory, 93 us like this.
 template <int L>
-__global__ void __launch_bounds__(VCfg<L>::NT, VCfg<L>::COLS_CTAS)
+__global__ void __launch_bounds__(ColFFT<L / 2>::NT, L <= 512 ? 512 / ColFFT<L / 2>::NT : 1)
 k_volkov_cols(const float2* __restrict__ zph, const float* __restrict__ gxh, const float2* __restrict__ tw,
               float2* __restrict__ cdct) {
-    using C = VCfg<L>;
-    using WF = typename C::WF;
-    constexpr int F = L / 2, NC = C::NC, NT = C::NT, FS = C::FS, T = WF::T, E = WF::E;
+    constexpr int F = L / 2;
+    using C = ColFFT<F>;
+    using W = typename C::W;
+    constexpr int T = W::T, E = W::E;
     extern __shared__ float2 sm[];
-    float2* sq = sm + C::BF * FS;  // NC arrays: gx + i (-1)^y gy of each column (permuted), then c[.][x]
-    const int a = blockIdx.y, x0 = blockIdx.x * NC;
-    const int tr = threadIdx.x / T, j = threadIdx.x % T;
-    auto src = [&](int y, int c) { return ((size_t)a * F + y) * F + x0 + c; };
-    // image row y goes to element m of the permuted column, mirror_pos(m) = y
-    auto slot = [&](int y) { return (y & 1) ? F - 1 - (y >> 1) : (y >> 1); };
-#pragma unroll  // every staging load in flight before the first store
-    for (int i = threadIdx.x; i < NC * F; i += NT) {
-        const int c = i % NC, y = i / NC;
-        const size_t o = src(y, c);
-        sm[c * FS + WF::pad(slot(y))] = zph[o];
-    }
-    __syncthreads();
-    {  // y derivatives of Z
-        float2* s = sm + tr * FS;
-        float2 x[E];
+    const int t = C::column();
+    const ColLanes<F> ln{sm + t * W::STRIDE, C::paired_j()};
+    const int j = ln.j;
+    const size_t o = (size_t)blockIdx.y * F * F + blockIdx.x * C::B + t;
+    float2 x[E];
 #pragma unroll
-        for (int n1 = 0; n1 < E; ++n1) x[n1] = s[WF::pad(j + n1 * T)];
-        mirror_derivative<F>(x, s, j, tw);
-        __syncwarp();
+    for (int n1 = 0; n1 < E; ++n1) x[n1] = zph[o + (size_t)mirror_pos(j + n1 * T, F) * F];
+    mirror_derivative<F>(x, ln, tw);
+    // gy = Re(-i dZ/dy / Z) / 2pi at Y = F + y
 #pragma unroll
-        for (int n1 = 0; n1 < E; ++n1) s[WF::pad(mirror_pos(j + n1 * T, F))] = x[n1];
-    }
-    __syncthreads();
-    // gy = Re(-i dZ/dy / Z) / 2pi at Y = F + y; the Q array takes
-    // gx + i (-1)^y gy, permuted (column_dct_dst's input)
-#pragma unroll 4
-    for (int i = threadIdx.x; i < NC * F; i += NT) {
-        const int c = i % NC, y = i / NC;
-        const size_t o = src(y, c);
-        const float2 z = zph[o];
-        const float gx = gxh[o];
-        const float2 g = sm[c * FS + WF::pad(y)];
+    for (int n1 = 0; n1 < E; ++n1) {
+        const int m = j + n1 * T;  // row mirror_pos(m): even for m < F/2
+        const size_t i = o + (size_t)mirror_pos(m, F) * F;
+        const float2 z = zph[i], g = x[n1];
         const float gy = (g.y * z.x - g.x * z.y) / (z.x * z.x + z.y * z.y) * kInvTwoPi;
-        sq[c * FS + WF::pad(slot(y))] = make_float2(gx, (y & 1) ? -gy : gy);
+        x[n1] = make_float2(gxh[i], m < F / 2 ? gy : -gy);
     }
-    __syncthreads();
-    {
-        float2* s = sq + tr * FS;
-        float2 x[E];
-#pragma unroll
-        for (int n1 = 0; n1 < E; ++n1) x[n1] = s[WF::pad(j + n1 * T)];
-        column_dct_dst<F>(x, s, j, tw, [&](int k, float2 v) { s[k] = v; });
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int i = threadIdx.x; i < NC * F; i += NT) {
-        const int c = i % NC, ky = i / NC;
-        cdct[((size_t)a * F + ky) * F + x0 + c] = sq[c * FS + ky];
-    }
+    column_dct_dst<F>(x, ln, tw, [&](int k, float2 v) { cdct[o + (size_t)k * F] = v; });
 }
 
 // Pass 3: rows ky of the Poisson solve: integ_grad4 on the mirror
@@ -406,7 +390,7 @@ template <int F>
 struct ICfg {
     using W = WarpFFT<F>;
     static constexpr int NW = 4;                   // warps per CTA
-    static constexpr int R = 2 * NW * W::G;        // rows (pass 3) or columns (pass 4) per CTA, two per transform
+    static constexpr int R = 2 * NW * W::G;        // rows per CTA, two per transform
     static constexpr int NT = NW * 32;
     static constexpr size_t SMEM = (size_t)NW * W::G * W::STRIDE * sizeof(float2);
 };
@@ -501,53 +485,38 @@ k_volkov_integ_rows(const float2* __restrict__ cdct, const float2* __restrict__ 
     }
 }
 
-// Pass 4: columns of U, two per transform: the DCT-III along y (dct3_input
-// and one inverse transform) gives the unwrapped phase less its mean, and the
-// wrapped phase's mean (from the field column pass's nps sums) is added as
-// the rows are stored, contiguous, through the transforms' arrays.
+// Pass 4: columns of U, two neighbouring ones per transform (ColFFT on pairs):
+// the DCT-III along y (dct3_input and one inverse transform) gives the
+// unwrapped phase less its mean, and the wrapped phase's mean (from the field
+// column pass's nps sums) is added as the rows are stored.
 template <int F>
-__global__ void __launch_bounds__(ICfg<F>::NT)
-k_volkov_integ_cols(const float* __restrict__ urows, const double* __restrict__ psum, int nps,
-                    const float2* __restrict__ tw, float* __restrict__ unwrapped) {
-    using C = ICfg<F>;
+__global__ void __launch_bounds__(ColFFT<F>::NT)
+k_volkov_integ_cols(const float2* __restrict__ urows, const double* __restrict__ psum, int nps,
+                    const float2* __restrict__ tw, float2* __restrict__ unwrapped) {
+    using C = ColFFT<F>;
     using W = typename C::W;
-    constexpr int T = W::T, E = W::E, L = 2 * F, R = C::R, NT = C::NT;
+    constexpr int T = W::T, E = W::E, L = 2 * F;
     extern __shared__ float2 sm[];
-    const int tr = threadIdx.x / T, j = threadIdx.x % T;
-    const int a = blockIdx.y, c0 = blockIdx.x * R;
-    float* smf = reinterpret_cast<float*>(sm);
+    const int t = C::column(), j = C::paired_j();
+    const size_t o = (size_t)blockIdx.y * F * (F / 2) + blockIdx.x * C::B + t;  // pairs of columns
     __shared__ float s_mean;
-    if (threadIdx.x == 0) s_mean = phase_mean(psum + (size_t)a * kPhaseParts, nps, F);  // ordered by the barrier below
-    // column c0 + t of U into float slot (t & 1) of transform t / 2's array, at row ky
-#pragma unroll  // every staging load in flight before the first store
-    for (int r = 0; r < R * F / NT; ++r) {
-        const int i = threadIdx.x + r * NT, t = i % R, ky = i / R;
-        smf[2 * ((t >> 1) * W::STRIDE + ky) + (t & 1)] = urows[((size_t)a * F + ky) * F + c0 + t];
-    }
-    __syncthreads();
-    float2* s = sm + tr * W::STRIDE;
-    const int src = ((threadIdx.x & 31) & ~(T - 1)) + ((T - j) & (T - 1));
-    float2 wl[E / T];
+    if (threadIdx.x == 0)  // ordered by the transform's barrier
+        s_mean = phase_mean(psum + (size_t)blockIdx.y * kPhaseParts, nps, F);
+    float2 wl[E / T];  // e^{-i pi (j + qT)/2F}
 #pragma unroll
     for (int q = 0; q < E / T; ++q) wl[q] = __ldg(&tw[(j + q * T) * (kTwN / (2 * L))]);
     float2 xv[E], y[E];
 #pragma unroll
     for (int q = 0; q < E / T; ++q) {
 #pragma unroll
-        for (int k2 = 0; k2 < T; ++k2) xv[q * T + k2] = s[j + q * T + E * k2];
+        for (int k2 = 0; k2 < T; ++k2) xv[q * T + k2] = urows[o + (size_t)(j + q * T + E * k2) * (F / 2)];
     }
-    dct3_input<F>(xv, wl, j, src, y);
-    fft_warp_regs_rev<F, +1>(y, s, j, tw);
-    __syncwarp();  // the transform's exchange is done with s
-#pragma unroll
-    for (int n1 = 0; n1 < E; ++n1) s[mirror_pos(j + n1 * T, F)] = y[n1];
-    __syncthreads();
+    dct3_input<F>(xv, wl, j, C::partner(), y);
+    fft_cta_regs_rev<F, +1>(y, sm + t * W::STRIDE, j, tw);
     const float mean = s_mean;
-#pragma unroll 8
-    for (int r = 0; r < R * F / NT; ++r) {
-        const int i = threadIdx.x + r * NT, t = i % R, yy = i / R;
-        unwrapped[((size_t)a * F + yy) * F + c0 + t] = mean + smf[2 * ((t >> 1) * W::STRIDE + yy) + (t & 1)];
-    }
+#pragma unroll
+    for (int n1 = 0; n1 < E; ++n1)
+        unwrapped[o + (size_t)mirror_pos(j + n1 * T, F) * (F / 2)] = make_float2(mean + y[n1].x, mean + y[n1].y);
 }
 
 // ---------------------------------------------------------------- aberration fit
@@ -642,18 +611,17 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
                 bool form) {
     constexpr int L = 2 * F;
     using FC = FieldCfg<F>;
-    using VC = VCfg<L>;
+    using CC = ColFFT<F>;
     using IC = ICfg<F>;
     const Params& p = c->p;
     Buffers& b = c->b;
     const size_t FF = (size_t)F * F;
-    static_assert(F / FC::B <= kPhaseParts, "phase sums per angle");
+    static_assert(F / CC::B <= kPhaseParts, "phase sums per angle");
     using RC = RCfg<F>;
     const size_t sm_vrows = RC::SMEM;
-    const size_t sm_vcols = VC::SMEM_COLS;
-    if (allow_smem(k_field_rows<F>, FC::SMEM) || allow_smem(k_field_cols<F>, FC::SMEM) ||
-        allow_smem(k_volkov_rows<L>, sm_vrows) || allow_smem(k_volkov_cols<L>, sm_vcols) ||
-        allow_smem(k_volkov_integ_rows<F>, IC::SMEM) || allow_smem(k_volkov_integ_cols<F>, IC::SMEM))
+    if (allow_smem(k_field_rows<F>, FC::SMEM) || allow_smem(k_field_cols<F>, CC::SMEM) ||
+        allow_smem(k_volkov_rows<L>, sm_vrows) || allow_smem(k_volkov_cols<L>, CC::SMEM) ||
+        allow_smem(k_volkov_integ_rows<F>, IC::SMEM) || allow_smem(k_volkov_integ_cols<F>, CC::SMEM))
         return TDM_ECUDA;
     const int step = angles_per_launch(c, n);
     for (int g0 = a0; g0 < a0 + n; g0 += step) {
@@ -672,8 +640,9 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
         }
         {
             Launch l(c, K_FIELD_COLS);
-            k_field_cols<F><<<dim3(F / FC::B, m), FC::NT, FC::SMEM, c->stream>>>(
-                b.I1, p.c_aber, b.tw, b.phase, b.amp, b.zph, b.fields + (size_t)g0 * FF, b.phase_sum);
+            const bool keep = dbg_phase || !(p.deroul && p.volkov);
+            k_field_cols<F><<<dim3(F / CC::B, m), CC::NT, CC::SMEM, c->stream>>>(
+                b.I1, p.c_aber, b.tw, keep ? b.phase : nullptr, b.amp, b.zph, b.fields + (size_t)g0 * FF, b.phase_sum);
         }
         if (!p.c_aber) continue;
         const float* unw = b.phase;
@@ -687,7 +656,7 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
             }
             {
                 Launch l(c, K_VOLKOV_COLS);
-                k_volkov_cols<L><<<dim3(F / VC::NC, m), VC::NT, sm_vcols, c->stream>>>(b.zph, b.gx, b.tw, b.qc);
+                k_volkov_cols<L><<<dim3(F / CC::B, m), CC::NT, CC::SMEM, c->stream>>>(b.zph, b.gx, b.tw, b.qc);
             }
             float* urows = reinterpret_cast<float*>(b.tq);
             {
@@ -696,8 +665,8 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
             }
             {
                 Launch l(c, K_VOLKOV_INTEG_COLS);
-                k_volkov_integ_cols<F><<<dim3(F / IC::R, m), IC::NT, IC::SMEM, c->stream>>>(
-                    urows, b.phase_sum, F / FC::B, b.tw, b.unwrapped);
+                k_volkov_integ_cols<F><<<dim3(F / 2 / CC::B, m), CC::NT, CC::SMEM, c->stream>>>(
+                    b.tq, b.phase_sum, F / CC::B, b.tw, reinterpret_cast<float2*>(b.unwrapped));
             }
             unw = b.unwrapped;
         }

@@ -416,11 +416,9 @@ gk_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, con
             const float* __restrict__ s_tabf, Params p, const float2* __restrict__ wq, float2* __restrict__ rec,
             int16_t* __restrict__ recz, int* __restrict__ err) {
     extern __shared__ float2 sm[];
-    __shared__ double s_fz;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int a = blockIdx.y, kx0 = blockIdx.x * kCols;
     const int2 ps = posspec[a];
-    if (threadIdx.x == 0) s_fz = cap_fzm0(p, ps);
     staged_copy<kCols * F, kCols * 32>(
         threadIdx.x,
         [&](int i) {
@@ -433,14 +431,14 @@ gk_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, con
     __syncthreads();
     if (kx0 + w < F) gfft<F, -1, 4 * F>(sm + w * 2 * F, sm + w * 2 * F + F, wq, lane);
     __syncthreads();
-    const double fz = s_fz;
-    const float fzf = (float)fz, ir = (float)p.inv_rayon;
+    const CapFz fz = cap_fzm0(p, ps, s_tab, s_tabf);
+    const float ir = (float)p.inv_rayon;
     for (int i = threadIdx.x; i < kCols * F; i += blockDim.x) {
         const int t = i % kCols, ky = i / kCols, kx = kx0 + t;
         if (kx >= F) continue;
         const size_t o = ((size_t)a * F + ky) * F + kx;
         float sf = 0.f;
-        const int z = cap_plane(p, ps, fz, fzf, kx, ky, s_tab, s_tabf, &sf, err);
+        const int z = cap_plane(p, ps, fz, kx, ky, s_tab, s_tabf, &sf, err);
         float2 val = make_float2(0.f, 0.f);
         if (z >= 0) {
             const float2 v = sm[t * 2 * F + ky];

@@ -112,44 +112,65 @@ k_cap_rows_form(const float* __restrict__ unwrapped, const float* __restrict__ a
     }
 }
 
+// Column passes (ColFFT) with at least 512 threads an SM: 128 registers each.
+template <int D>
+struct ColPass : ColFFT<D> {
+    using ColFFT<D>::NT;
+    static constexpr int CTAS = NT <= 128 ? 4 : NT <= 256 ? 2 : 1;
+};
+
+// Columns of the per-field spectrum (ColFFT) and their cap records.
 template <int F>
-__global__ void __launch_bounds__(CapCfg<F>::NT)
+__global__ void __launch_bounds__(ColFFT<F>::NT, 512 / ColFFT<F>::NT)
 k_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, const double* __restrict__ s_tab,
            const float* __restrict__ s_tabf, Params p, const float2* __restrict__ tw, float2* __restrict__ rec,
            int16_t* __restrict__ recz, int* __restrict__ err) {
-    using C = CapCfg<F>;
+    using C = ColFFT<F>;
     using W = typename C::W;
-    constexpr int B = C::B, NT = C::NT;
+    constexpr int T = W::T, E = W::E;
     extern __shared__ float2 sm[];
-    __shared__ double s_fz;
-    const int tr = threadIdx.x / W::T, j = threadIdx.x % W::T;
-    const int a = blockIdx.y, kx0 = blockIdx.x * B;
+    const int t = C::column(), j = C::adjacent_j();
+    const int a = blockIdx.y, kx = blockIdx.x * C::B + t;
     const int2 ps = posspec[a];
-    if (threadIdx.x == 0) s_fz = cap_fzm0(p, ps);
-#pragma unroll  // every load in flight before the first store
-    for (int r = 0; r < B * F / NT; ++r) {
-        const int i = threadIdx.x + r * NT, t = i % B, ky = i / B;
-        sm[t * W::STRIDE + W::pad(ky)] = r1[((size_t)a * F + ky) * F + kx0 + t];
-    }
-    __syncthreads();
-    fft_warp<F, -1>(sm + tr * W::STRIDE, j, tw);
-    __syncthreads();
-    const double fz = s_fz;
-    const float fzf = (float)fz, ir = (float)p.inv_rayon;
-#pragma unroll 2
-    for (int r = 0; r < B * F / NT; ++r) {
-        const int i = threadIdx.x + r * NT, t = i % B, ky = i / B, kx = kx0 + t;
-        const size_t o = ((size_t)a * F + ky) * F + kx;
+    const CapFz fz = cap_fzm0(p, ps, s_tab, s_tabf);
+    const float ir = (float)p.inv_rayon;
+    const size_t o = (size_t)a * F * F + kx;
+    float2 x[E];
+#pragma unroll
+    for (int n1 = 0; n1 < E; ++n1) x[n1] = r1[o + (size_t)(j + n1 * T) * F];
+    fft_cta_regs<F, -1>(x, sm + t * W::STRIDE, j, tw);
+    auto put = [&](int ky, float2 v) {
         float sf = 0.f;
-        const int z = cap_plane(p, ps, fz, fzf, kx, ky, s_tab, s_tabf, &sf, err);
+        const int z = cap_plane(p, ps, fz, kx, ky, s_tab, s_tabf, &sf, err);
         float2 val = make_float2(0.f, 0.f);
         if (z >= 0) {
-            const float2 v = sm[t * W::STRIDE + W::pad(ky)];
             const float Bc = cap_weight(p, sf, ir, kx, ky);
             val = make_float2(-Bc * v.y, Bc * v.x);
         }
-        rec[o] = val;
-        recz[o] = (int16_t)z;
+        rec[o + (size_t)ky * F] = val;
+        recz[o + (size_t)ky * F] = (int16_t)z;
+    };
+    if constexpr (E <= 16) {
+#pragma unroll
+        for (int q = 0; q < E / T; ++q) {
+#pragma unroll
+            for (int k2 = 0; k2 < T; ++k2) put(j + q * T + E * k2, x[q * T + k2]);
+        }
+    } else {
+        // 32 unrolled bins take 246 registers (194 us for 64 angles of 512^2, against 148 as below): the
+        // thread's values wait in its own places of the exchange array instead
+        float2* s = sm + t * W::STRIDE;
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < E / T; ++q) {
+#pragma unroll
+            for (int k2 = 0; k2 < T; ++k2) s[warp_out_pos<F>(j, q, k2)] = x[q * T + k2];
+        }
+#pragma unroll 2
+        for (int i = 0; i < E; ++i) {
+            const int q = i / T, k2 = i % T;
+            put(j + q * T + E * k2, s[warp_out_pos<F>(j, q, k2)]);
+        }
     }
 }
 
@@ -379,26 +400,11 @@ k_gather(const float2* __restrict__ rec, const int16_t* __restrict__ recz, const
 }
 
 // ---------------------------------------------------------------- 3D FFT passes
-// Column passes (y, z): a CTA transforms B consecutive x.  The T threads of
-// a transform sit B apart, so a warp's lanes are consecutive x (of two
-// neighbouring elements): loads and stores go straight between registers and
-// global memory in 128-byte lines, and shared memory holds the FFT's one
-// transposing exchange only, with a CTA barrier around it.  (A warp per
-// transform, with the columns staged and unstaged through shared memory, took
-// three times the shared-memory traffic and bounded the passes.)  Bound by HBM:
-// 512^3 with a band of 220, x 137 us and y 144 us (6.7 and 6.4 TB/s), z 337 us
-// (4.5 TB/s, most of it stores); over all planes y and x took 405 and 432 us.
-// B = 8 leaves 32-byte pieces in the z pass's stores (713 us), B = 32 one CTA an
-// SM (y 182, z 352 us).
-template <int D>
-struct ColPass {
-    using W = WarpFFT<D>;
-    static constexpr int B = 16;
-    static constexpr int NT = B * W::T;
-    static constexpr size_t SMEM = (size_t)B * W::STRIDE * sizeof(float2);
-    static constexpr int CTAS = NT <= 128 ? 4 : NT <= 256 ? 2 : 1;  // 128 registers a thread
-};
-
+// Column passes (y, z): ColFFT, 16 consecutive x a CTA.  Bound by HBM: 512^3
+// with a band of 220, x 137 us and y 144 us (6.7 and 6.4 TB/s), z 337 us
+// (4.5 TB/s, most of it stores); over all planes and staged through shared memory
+// y and x took 405 and 432 us.  8 columns leave 32-byte pieces in the z pass's
+// stores (713 us), 32 one CTA an SM (y 182, z 352 us).
 // Row pass (x): a warp per G rows, registers to registers.
 template <int D>
 struct RowPass {
@@ -455,7 +461,7 @@ k_ypass(float2* __restrict__ vol, const float2* __restrict__ tw, Params p) {
     using W = typename C::W;
     constexpr int T = W::T, E = W::E;
     extern __shared__ float2 sm[];
-    const int t = threadIdx.x % C::B, j = threadIdx.x / C::B;
+    const int t = C::column(), j = C::adjacent_j();
     float2* col = vol + (size_t)blockIdx.y * D * D + blockIdx.x * C::B + t;
     float2 x[E];
 #pragma unroll
@@ -485,7 +491,7 @@ k_zpass(const float2* __restrict__ vol, const float2* __restrict__ tw, Params p,
     using W = typename C::W;
     constexpr int T = W::T, E = W::E;
     extern __shared__ float2 sm[];
-    const int t = threadIdx.x % C::B, j = threadIdx.x / C::B;
+    const int t = C::column(), j = C::adjacent_j();
     const int X = blockIdx.x * C::B + t, Y = y0 + blockIdx.y;
     const float2* col = vol + (size_t)Y * D + X;
     float2 x[E];
@@ -528,7 +534,7 @@ k_fzpass(const float* __restrict__ re, const float* __restrict__ im, const float
     using W = typename C::W;
     constexpr int T = W::T, E = W::E;
     extern __shared__ float2 sm[];
-    const int t = threadIdx.x % C::B, j = threadIdx.x / C::B;
+    const int t = C::column(), j = C::adjacent_j();
     const int X = blockIdx.x * C::B + t, Y = blockIdx.y;
     const size_t o = (size_t)Y * D + X;
     const float sg = ((X + Y + j + 3 * (D / 2)) & 1) ? -scale : scale;  // z has j's parity
@@ -560,18 +566,14 @@ k_cap_sample(const float2* __restrict__ vol, const int2* __restrict__ posspec, P
              int* __restrict__ err) {
     const int a = blockIdx.y, F = p.F, D = p.D;
     const int2 ps = posspec[a];
-    __shared__ double s_fz;
     __shared__ double red[8];
-    if (threadIdx.x == 0) s_fz = cap_fzm0(p, ps);
-    __syncthreads();
-    const double fz = s_fz;
-    const float fzf = (float)fz;
+    const CapFz fz = cap_fzm0(p, ps, s_tab, s_tabf);
     double m2 = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < F * F; i += gridDim.x * blockDim.x) {
         const int kx = i % F, ky = i / F;
         const size_t o = (size_t)a * F * F + i;
         float sf;
-        const int z = cap_plane(p, ps, fz, fzf, kx, ky, s_tab, s_tabf, &sf, err);
+        const int z = cap_plane(p, ps, fz, kx, ky, s_tab, s_tabf, &sf, err);
         float2 v = make_float2(0.f, 0.f);
         if (z >= 0) {
             const float2 d = data ? data[o] : make_float2(0.f, 0.f);
@@ -606,15 +608,11 @@ k_cap_pack(const float2* __restrict__ caps, const int2* __restrict__ posspec, Pa
            int16_t* __restrict__ recz, int* __restrict__ err) {
     const int a = blockIdx.y, F = p.F;
     const int2 ps = posspec[a];
-    __shared__ double s_fz;
-    if (threadIdx.x == 0) s_fz = cap_fzm0(p, ps);
-    __syncthreads();
-    const double fz = s_fz;
-    const float fzf = (float)fz;
+    const CapFz fz = cap_fzm0(p, ps, s_tab, s_tabf);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < F * F; i += gridDim.x * blockDim.x) {
         const size_t o = (size_t)a * F * F + i;
         float sf;
-        const int z = cap_plane(p, ps, fz, fzf, i % F, i / F, s_tab, s_tabf, &sf, err);
+        const int z = cap_plane(p, ps, fz, i % F, i / F, s_tab, s_tabf, &sf, err);
         const float2 v = z >= 0 ? caps[o] : make_float2(0.f, 0.f);
         rec[o] = v;
         recz[o] = (int16_t)z;
@@ -743,7 +741,7 @@ int cap_impl(tdm_ctx* c, int a0, int n, bool form) {
     using C = CapCfg<F>;
     Buffers& b = c->b;
     if (allow_smem(k_cap_rows<F>, C::SMEM) || allow_smem(k_cap_rows_form<F>, C::SMEM) ||
-        allow_smem(k_cap_cols<F>, C::SMEM))
+        allow_smem(k_cap_cols<F>, ColFFT<F>::SMEM))
         return TDM_ECUDA;
     if (form && n > c->chunk) return TDM_EINVAL;  // the chunk buffers hold one chunk
     const size_t FF = (size_t)F * F;
@@ -762,7 +760,8 @@ int cap_impl(tdm_ctx* c, int a0, int n, bool form) {
         }
         {
             Launch l(c, K_CAP_COLS);
-            k_cap_cols<F><<<dim3(F / C::B, m), C::NT, C::SMEM, c->stream>>>(
+            using CC = ColFFT<F>;
+            k_cap_cols<F><<<dim3(F / CC::B, m), CC::NT, CC::SMEM, c->stream>>>(
                 b.r1, b.posspec + g0, b.s_tab, b.s_tabf, c->p, b.tw, b.rec.val + g0 * FF, b.rec.z + g0 * FF, b.err);
         }
     }
