@@ -413,7 +413,7 @@ gk_cap_rows(const float2* __restrict__ fields_in, const float* __restrict__ unwr
 template <int F>
 __global__ void __launch_bounds__(kCols * 32)
 gk_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, const double* __restrict__ s_tab,
-            const float* __restrict__ s_tabf, Params p, const float2* __restrict__ wq, float2* __restrict__ rec,
+            const float2* __restrict__ s_pair, Params p, const float2* __restrict__ wq, float2* __restrict__ rec,
             int16_t* __restrict__ recz, int* __restrict__ err) {
     extern __shared__ float2 sm[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -431,14 +431,14 @@ gk_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, con
     __syncthreads();
     if (kx0 + w < F) gfft<F, -1, 4 * F>(sm + w * 2 * F, sm + w * 2 * F + F, wq, lane);
     __syncthreads();
-    const CapFz fz = cap_fzm0(p, ps, s_tab, s_tabf);
+    const CapFz fz = cap_fzm0(p, ps, s_tab, s_pair);
     const float ir = (float)p.inv_rayon;
     for (int i = threadIdx.x; i < kCols * F; i += blockDim.x) {
         const int t = i % kCols, ky = i / kCols, kx = kx0 + t;
         if (kx >= F) continue;
         const size_t o = ((size_t)a * F + ky) * F + kx;
         float sf = 0.f;
-        const int z = cap_plane(p, ps, fz, kx, ky, s_tab, s_tabf, &sf, err);
+        const int z = cap_plane(p, ps, fz, kx, ky, s_tab, s_pair, &sf, err);
         float2 val = make_float2(0.f, 0.f);
         if (z >= 0) {
             const float2 v = sm[t * 2 * F + ky];
@@ -547,7 +547,7 @@ int gcap_impl(tdm_ctx* c, int a0, int n, bool form) {
         }
         {
             Launch l(c, K_CAP_COLS);
-            gk_cap_cols<F><<<dim3(cols, m), kCols * 32, sm_cols, c->stream>>>(b.r1, b.posspec + g0, b.s_tab, b.s_tabf,
+            gk_cap_cols<F><<<dim3(cols, m), kCols * 32, sm_cols, c->stream>>>(b.r1, b.posspec + g0, b.s_tab, b.s_pair,
                                                                             c->p, b.wq, b.rec.val + g0 * FF,
                                                                             b.rec.z + g0 * FF, b.err);
         }

@@ -123,7 +123,7 @@ struct ColPass : ColFFT<D> {
 template <int F>
 __global__ void __launch_bounds__(ColFFT<F>::NT, 512 / ColFFT<F>::NT)
 k_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, const double* __restrict__ s_tab,
-           const float* __restrict__ s_tabf, Params p, const float2* __restrict__ tw, float2* __restrict__ rec,
+           const float2* __restrict__ s_pair, Params p, const float2* __restrict__ tw, float2* __restrict__ rec,
            int16_t* __restrict__ recz, int* __restrict__ err) {
     using C = ColFFT<F>;
     using W = typename C::W;
@@ -132,7 +132,7 @@ k_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, cons
     const int t = C::column(), j = C::adjacent_j();
     const int a = blockIdx.y, kx = blockIdx.x * C::B + t;
     const int2 ps = posspec[a];
-    const CapFz fz = cap_fzm0(p, ps, s_tab, s_tabf);
+    const CapFz fz = cap_fzm0(p, ps, s_tab, s_pair);
     const float ir = (float)p.inv_rayon;
     const size_t o = (size_t)a * F * F + kx;
     float2 x[E];
@@ -141,7 +141,7 @@ k_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, cons
     fft_cta_regs<F, -1>(x, sm + t * W::STRIDE, j, tw);
     auto put = [&](int ky, float2 v) {
         float sf = 0.f;
-        const int z = cap_plane(p, ps, fz, kx, ky, s_tab, s_tabf, &sf, err);
+        const int z = cap_plane(p, ps, fz, kx, ky, s_tab, s_pair, &sf, err);
         float2 val = make_float2(0.f, 0.f);
         if (z >= 0) {
             const float Bc = cap_weight(p, sf, ir, kx, ky);
@@ -561,26 +561,27 @@ k_fzpass(const float* __restrict__ re, const float* __restrict__ im, const float
 // sum |residual|^2 added to *misfit.
 __global__ void __launch_bounds__(256)
 k_cap_sample(const float2* __restrict__ vol, const int2* __restrict__ posspec, Params p,
-             const double* __restrict__ s_tab, const float* __restrict__ s_tabf, const float2* __restrict__ data,
+             const double* __restrict__ s_tab, const float2* __restrict__ s_pair, const float2* __restrict__ data,
              float2* __restrict__ caps, float2* __restrict__ res, int16_t* __restrict__ resz, double* __restrict__ misfit,
              int* __restrict__ err) {
     const int a = blockIdx.y, F = p.F, D = p.D;
     const int2 ps = posspec[a];
     __shared__ double red[8];
-    const CapFz fz = cap_fzm0(p, ps, s_tab, s_tabf);
+    const CapFz fz = cap_fzm0(p, ps, s_tab, s_pair);
     double m2 = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < F * F; i += gridDim.x * blockDim.x) {
         const int kx = i % F, ky = i / F;
         const size_t o = (size_t)a * F * F + i;
         float sf;
-        const int z = cap_plane(p, ps, fz, kx, ky, s_tab, s_tabf, &sf, err);
+        const int z = cap_plane(p, ps, fz, kx, ky, s_tab, s_pair, &sf, err);
         float2 v = make_float2(0.f, 0.f);
         if (z >= 0) {
             const float2 d = data ? data[o] : make_float2(0.f, 0.f);
             const int X = cap_col(p, kx, ps.x), Y = cap_col(p, ky, ps.y);
             v = vol[((size_t)(z - p.zmin) * D + Y) * D + X];
             v = make_float2(v.x - d.x, v.y - d.y);
-            m2 += (double)v.x * v.x + (double)v.y * v.y;
+            const double vx = widen(v.x), vy = widen(v.y);  // the FP64 pipe squares and adds only
+            m2 = fma(vy, vy, fma(vx, vx, m2));
         }
         if (caps) caps[o] = v;
         if (res) {
@@ -604,15 +605,15 @@ k_cap_sample(const float2* __restrict__ vol, const int2* __restrict__ posspec, P
 // Cap values of given values on the cap cells (0 elsewhere), for the scatter.
 __global__ void __launch_bounds__(256)
 k_cap_pack(const float2* __restrict__ caps, const int2* __restrict__ posspec, Params p,
-           const double* __restrict__ s_tab, const float* __restrict__ s_tabf, float2* __restrict__ rec,
+           const double* __restrict__ s_tab, const float2* __restrict__ s_pair, float2* __restrict__ rec,
            int16_t* __restrict__ recz, int* __restrict__ err) {
     const int a = blockIdx.y, F = p.F;
     const int2 ps = posspec[a];
-    const CapFz fz = cap_fzm0(p, ps, s_tab, s_tabf);
+    const CapFz fz = cap_fzm0(p, ps, s_tab, s_pair);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < F * F; i += gridDim.x * blockDim.x) {
         const size_t o = (size_t)a * F * F + i;
         float sf;
-        const int z = cap_plane(p, ps, fz, i % F, i / F, s_tab, s_tabf, &sf, err);
+        const int z = cap_plane(p, ps, fz, i % F, i / F, s_tab, s_pair, &sf, err);
         const float2 v = z >= 0 ? caps[o] : make_float2(0.f, 0.f);
         rec[o] = v;
         recz[o] = (int16_t)z;
@@ -762,7 +763,7 @@ int cap_impl(tdm_ctx* c, int a0, int n, bool form) {
             Launch l(c, K_CAP_COLS);
             using CC = ColFFT<F>;
             k_cap_cols<F><<<dim3(F / CC::B, m), CC::NT, CC::SMEM, c->stream>>>(
-                b.r1, b.posspec + g0, b.s_tab, b.s_tabf, c->p, b.tw, b.rec.val + g0 * FF, b.rec.z + g0 * FF, b.err);
+                b.r1, b.posspec + g0, b.s_tab, b.s_pair, c->p, b.tw, b.rec.val + g0 * FF, b.rec.z + g0 * FF, b.err);
         }
     }
     return cudaGetLastError() == cudaSuccess ? TDM_OK : TDM_ECUDA;
@@ -904,7 +905,7 @@ int forward_impl(tdm_ctx* c, const float* xn, const float* xk, int n, float2* ca
     {
         Launch l(c, K_CAP_COLS);
         const int per = (p.F * p.F + 255) / 256;
-        k_cap_sample<<<dim3(per < 16 ? per : 16, n), 256, 0, c->stream>>>(b.vol, b.posspec, p, b.s_tab, b.s_tabf, data,
+        k_cap_sample<<<dim3(per < 16 ? per : 16, n), 256, 0, c->stream>>>(b.vol, b.posspec, p, b.s_tab, b.s_pair, data,
                                                                           caps, res.val, res.z, misfit, b.err);
     }
     return cudaGetLastError() == cudaSuccess ? TDM_OK : TDM_ECUDA;
@@ -989,7 +990,7 @@ int launch_cap_pack(tdm_ctx* c, const float2* caps, int n, CapRecs recs) {
     {
         Launch l(c, K_CAP_COLS);
         k_cap_pack<<<dim3(per < 16 ? per : 16, n), 256, 0, c->stream>>>(caps, c->b.posspec, c->p, c->b.s_tab,
-                                                                        c->b.s_tabf, recs.val, recs.z, c->b.err);
+                                                                        c->b.s_pair, recs.val, recs.z, c->b.err);
     }
     return cudaGetLastError() == cudaSuccess ? TDM_OK : TDM_ECUDA;
 }

@@ -95,7 +95,7 @@ int dev_alloc(tdm_ctx* c, T** p, size_t count) {
 
 void free_all(tdm_ctx* c) {
     Buffers& b = c->b;
-    void* ptrs[] = {b.tw, b.win_h, b.tuk_f, b.s_tab, b.s_tabf, b.wq, b.holo_stage, b.inter, b.spectra, b.posspec,
+    void* ptrs[] = {b.tw, b.win_h, b.tuk_f, b.s_tab, b.s_pair, b.wq, b.holo_stage, b.inter, b.spectra, b.posspec,
                     b.specval, b.argpart, b.I1, b.phase, b.amp, b.zph, b.gx, b.qc, b.tq, b.phase_sum, b.unwrapped, b.beta,
                     b.fit_part, b.fit_done, b.fields, b.r1, b.rec_buf[0].val, b.rec_buf[0].z, b.rec_buf[1].val,
                     b.rec_buf[1].z, b.posspec_vol[0], b.posspec_vol[1], b.vol, b.out_re, b.out_im, b.out_otf,
@@ -373,7 +373,7 @@ int tdm_create(const tdm_geom* geom, int max_angles, tdm_ctx** out) {
     TRY(dev_alloc(c, &b.win_h, p.H));
     TRY(dev_alloc(c, &b.tuk_f, F));
     TRY(dev_alloc(c, &b.s_tab, FF));
-    TRY(dev_alloc(c, &b.s_tabf, FF));
+    TRY(dev_alloc(c, &b.s_pair, FF));
     TRY(dev_alloc(c, &b.wq, 4 * F));
     TRY(dev_alloc(c, &b.holo_stage, 2 * CH * p.H * p.H * 2));
     TRY(dev_alloc(c, &b.inter, CH * p.H * F));
@@ -412,7 +412,11 @@ int tdm_create(const tdm_geom* geom, int max_angles, tdm_ctx** out) {
     c->tuk_h_flat = tukey_flat(p.H, 0.05f);
     c->tuk_f_flat = tukey_flat(F, 0.1f);
     std::vector<float> tff(tf.begin(), tf.end());
-    std::vector<float> stabf(stab.begin(), stab.end());
+    std::vector<float2> pairs(FF);  // the same as sums of two floats
+    for (size_t i = 0; i < FF; ++i) {
+        pairs[i].x = (float)stab[i];
+        pairs[i].y = (float)(stab[i] - (double)pairs[i].x);
+    }
     std::vector<float2> wq(4 * F);  // exp(-2 pi i k / 4F), for the mixed-radix passes
     for (int k = 0; k < 4 * F; ++k) {
         const double ang = -2.0 * M_PI * (double)k / (4.0 * F);
@@ -422,7 +426,7 @@ int tdm_create(const tdm_geom* geom, int max_angles, tdm_ctx** out) {
         cudaMemcpy(b.win_h, wh.data(), p.H * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(b.tuk_f, tff.data(), F * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(b.s_tab, stab.data(), FF * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(b.s_tabf, stabf.data(), FF * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(b.s_pair, pairs.data(), FF * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(b.wq, wq.data(), 4 * F * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(b.err, 0, 4 * sizeof(int)) != cudaSuccess ||
         cudaMemset(b.fit_done, 0, CH * 2 * sizeof(unsigned)) != cudaSuccess)

@@ -55,7 +55,7 @@ struct Buffers {
     float* ref_inv = nullptr;      // H*H, 1 / reference amplitude (tdm_set_reference_intensity), on first use
     float* tuk_f = nullptr;        // F, field Tukey alpha 0.1 (1D factor)
     double* s_tab = nullptr;       // F*F, sqrt(rayon^2 - fd^2) at [fdy+N][fdx+N]
-    float* s_tabf = nullptr;       // float copy
+    float2* s_pair = nullptr;      // the same values as pairs of floats (x the nearest float, x + y the value)
     float2* wq = nullptr;          // 4F, exp(-2 pi i k / 4F): twiddles of the mixed-radix passes
     uint8_t* holo_stage = nullptr; // host staging: 2 x chunk x H*H*2 bytes
     float2* inter = nullptr;       // chunk x F x H (extraction row pass, kx band column-major)
