@@ -117,13 +117,43 @@ k_field_rows(const float2* __restrict__ spectra, const float4* __restrict__ argp
     }
 }
 
-// Columns (ColFFT).  mode 1: phase/amplitude (C_ABER); mode 0: the field
-// itself is the result.  mode 1 also leaves the CTA's sum of the wrapped phase in
-// psum[a * kPhaseParts + blockIdx.x] (FP32 per thread and warp, FP64 across
-// the warps in a fixed order).  phase may be null (Volkov: only the sum is used).
-template <int F>
+// Amplitude |u| and unit phasor u/|u| (1 where u = 0: atan2(0, 0) = 0) from one
+// reciprocal square root: |u|^2 r, corrected by a Newton step of the square
+// root, and u r.  A field value whose square leaves the normal range is scaled
+// first.
+__device__ __forceinline__ float amplitude(float2 u, float2& z) {
+    auto unit = [&](float2 w) {
+        const float m2 = fmaf(w.x, w.x, w.y * w.y), r = rsqrtf(m2), m = m2 * r;
+        z = make_float2(w.x * r, w.y * r);
+        return fmaf(fmaf(-m, m, m2), 0.5f * r, m);
+    };
+    const float m2 = fmaf(u.x, u.x, u.y * u.y);
+    if (m2 > 1e-30f && m2 < 1e30f) return unit(u);
+    const float m = hypotf(u.x, u.y);
+    if (m > 0.0f && m < __int_as_float(0x7f800000)) {
+        const float k = m < 1.0f ? 0x1p100f : 0x1p-100f;
+        unit(make_float2(u.x * k, u.y * k));
+    } else {
+        z = m == 0.0f ? make_float2(1.0f, 0.0f) : make_float2(u.x / m, u.y / m);
+    }
+    return m;
+}
+
+// What the column pass leaves per field pixel.  FIELD (C_ABER off): the field
+// itself is the result.  The rest leave the amplitude and, for Volkov, the unit
+// phasor; for Herraez or no unwrapping, the wrapped phase.  Volkov's solve
+// gives the unwrapped phase less the wrapped phase's mean, a constant that the
+// aberration fit's constant term takes out of the field, so the phase is formed
+// only where the unwrapped phase itself is wanted (VOLKOV_PHASE), with each CTA's
+// sum of it in psum[a * kPhaseParts + blockIdx.x] (FP32 per thread and warp, FP64
+// across the warps in a fixed order).
+enum FieldMode { FIELD, PHASE, VOLKOV, VOLKOV_PHASE };
+
+// Columns (ColFFT).  Bound by issue: 100 angles of 256^2 35 us with atan2, hypot
+// and two divisions a pixel, 22 us as VOLKOV.
+template <int F, int MODE>
 __global__ void __launch_bounds__(ColFFT<F>::NT)
-k_field_cols(const float2* __restrict__ I1, int mode, const float2* __restrict__ tw, float* __restrict__ phase,
+k_field_cols(const float2* __restrict__ I1, const float2* __restrict__ tw, float* __restrict__ phase,
              float* __restrict__ amp, float2* __restrict__ zph, float2* __restrict__ fields,
              double* __restrict__ psum) {
     using C = ColFFT<F>;
@@ -145,20 +175,21 @@ k_field_cols(const float2* __restrict__ I1, int mode, const float2* __restrict__
             const float2 u = x[q * T + k2];
             const int yo = (j + q * T + E * k2 + F / 2) & (F - 1);
             const size_t o = ((size_t)a * F + yo) * F + xo;
-            if (mode) {
-                const float m = hypotf(u.x, u.y);
-                const float ph = atan2f(u.y, u.x);
-                if (phase) phase[o] = ph;
-                acc += ph;
-                amp[o] = m;
-                // exp(i phase) without the round trip through the angle; atan2(0, 0) = 0
-                zph[o] = m > 0.0f ? make_float2(u.x / m, u.y / m) : make_float2(1.0f, 0.0f);
-            } else {
+            if constexpr (MODE == FIELD) {
                 fields[o] = u;
+            } else {
+                float2 z;
+                amp[o] = amplitude(u, z);
+                if constexpr (MODE != PHASE) zph[o] = z;
+                if constexpr (MODE != VOLKOV) {
+                    const float ph = atan2f(u.y, u.x);
+                    phase[o] = ph;
+                    acc += ph;
+                }
             }
         }
     }
-    if (mode) phase_sum_cta<C::NT>(acc, psum + (size_t)a * kPhaseParts + blockIdx.x);
+    if constexpr (MODE == VOLKOV_PHASE) phase_sum_cta<C::NT>(acc, psum + (size_t)a * kPhaseParts + blockIdx.x);
 }
 
 // ---------------------------------------------------------------- Volkov unwrap
@@ -295,6 +326,13 @@ struct RCfg {
     static constexpr size_t SMEM = (size_t)B * W::STRIDE * sizeof(float2);
 };
 
+// Re(-i g / Z) / 2pi for a unit phasor Z: g conj(Z) / |Z|^2, where |Z|^2 = 1 + d
+// with d a few roundings, so 1 / |Z|^2 is 2 - |Z|^2 to d^2 (the division took a
+// fifth of the row pass: 100 angles of 256^2 32 -> 27 us).
+__device__ __forceinline__ float phasor_gradient(float2 g, float2 z) {
+    return (g.y * z.x - g.x * z.y) * (2.0f - fmaf(z.x, z.x, z.y * z.y)) * kInvTwoPi;
+}
+
 // Pass 1: rows of the mirror.  Mirror rows Y and L-1-Y are the same image
 // row, and only the right half of the phasor's gradient
 // gx = Re(-i dZ/dx / Z) / 2pi is kept: gx[Y][X] = sign(X) gxh[m(Y)][m(X)].
@@ -327,7 +365,7 @@ k_volkov_rows(const float2* __restrict__ zph, const float2* __restrict__ tw, flo
         const int xx = j + n1 * T;
         const float2 z = zr[xx];
         const float2 g = s[W::pad(xx)];
-        out[xx] = (g.y * z.x - g.x * z.y) / (z.x * z.x + z.y * z.y) * kInvTwoPi;  // Re(-i g / Z) / 2pi
+        out[xx] = phasor_gradient(g, z);
     }
 }
 
@@ -364,7 +402,7 @@ k_volkov_cols(const float2* __restrict__ zph, const float* __restrict__ gxh, con
         const int m = j + n1 * T;  // row mirror_pos(m): even for m < F/2
         const size_t i = o + (size_t)mirror_pos(m, F) * F;
         const float2 z = zph[i], g = x[n1];
-        const float gy = (g.y * z.x - g.x * z.y) / (z.x * z.x + z.y * z.y) * kInvTwoPi;
+        const float gy = phasor_gradient(g, z);
         x[n1] = make_float2(gxh[i], m < F / 2 ? gy : -gy);
     }
     column_dct_dst<F>(x, ln, tw, [&](int k, float2 v) { cdct[o + (size_t)k * F] = v; });
@@ -488,7 +526,7 @@ k_volkov_integ_rows(const float2* __restrict__ cdct, const float2* __restrict__ 
 // Pass 4: columns of U, two neighbouring ones per transform (ColFFT on pairs):
 // the DCT-III along y (dct3_input and one inverse transform) gives the
 // unwrapped phase less its mean, and the wrapped phase's mean (from the field
-// column pass's nps sums) is added as the rows are stored.
+// column pass's nps sums; nps = 0: left out) is added as the rows are stored.
 template <int F>
 __global__ void __launch_bounds__(ColFFT<F>::NT)
 k_volkov_integ_cols(const float2* __restrict__ urows, const double* __restrict__ psum, int nps,
@@ -501,7 +539,7 @@ k_volkov_integ_cols(const float2* __restrict__ urows, const double* __restrict__
     const size_t o = (size_t)blockIdx.y * F * (F / 2) + blockIdx.x * C::B + t;  // pairs of columns
     __shared__ float s_mean;
     if (threadIdx.x == 0)  // ordered by the transform's barrier
-        s_mean = phase_mean(psum + (size_t)blockIdx.y * kPhaseParts, nps, F);
+        s_mean = nps ? phase_mean(psum + (size_t)blockIdx.y * kPhaseParts, nps, F) : 0.0f;
     float2 wl[E / T];  // e^{-i pi (j + qT)/2F}
 #pragma unroll
     for (int q = 0; q < E / T; ++q) wl[q] = __ldg(&tw[(j + q * T) * (kTwN / (2 * L))]);
@@ -591,19 +629,23 @@ __global__ void __launch_bounds__(kFitThreads) k_aber_fit(const float* __restric
     if (threadIdx.x == 0) done[g] = 0;  // ready for the next chunk
 }
 
-// Evaluates the fits, corrects phase and amplitude and forms the Born or Rytov field.
-__global__ void __launch_bounds__(256) k_form(const float* __restrict__ unwrapped, const float* __restrict__ amp,
-                                              const double* __restrict__ beta, int F, int born,
-                                              float2* __restrict__ fields) {
-    const int a = blockIdx.y;
+// Evaluates the fits, corrects phase and amplitude and forms the Born or Rytov
+// field: a warp per row, so that the fits are reduced to polynomials in x once
+// for the row's F pixels (100 angles of 256^2: 34 us; per pixel 46).
+constexpr int kFormRows = 8;  // rows (warps) per CTA
+__global__ void __launch_bounds__(32 * kFormRows)
+k_form(const float* __restrict__ unwrapped, const float* __restrict__ amp, const double* __restrict__ beta, int F,
+       int born, float2* __restrict__ fields) {
+    const int a = blockIdx.y, y = blockIdx.x * kFormRows + (threadIdx.x >> 5);
     __shared__ float bf[2 * kNC];
     if (threadIdx.x < 2 * kNC) bf[threadIdx.x] = (float)beta[(size_t)a * 2 * kNC + threadIdx.x];
     __syncthreads();
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= F * F) return;
-    const int x = idx % F, y = idx / F;
-    const size_t o = (size_t)a * F * F + idx;
-    fields[o] = form_value(form_row(bf, y, F), x, F, unwrapped[o], amp[o], born);
+    if (y >= F) return;
+    const FormRow r = form_row(bf, y, F);
+    const size_t row = ((size_t)a * F + y) * F;
+#pragma unroll 4
+    for (int x = threadIdx.x & 31; x < F; x += 32)
+        fields[row + x] = form_value(r, x, F, unwrapped[row + x], amp[row + x], born);
 }
 
 template <int F>
@@ -617,9 +659,12 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
     Buffers& b = c->b;
     const size_t FF = (size_t)F * F;
     static_assert(F / CC::B <= kPhaseParts, "phase sums per angle");
+    const bool volkov = p.deroul && p.volkov, mean = volkov && (dbg_phase || dbg_unwrapped);
+    auto field_cols = !p.c_aber ? k_field_cols<F, FIELD> : mean ? k_field_cols<F, VOLKOV_PHASE>
+                      : volkov ? k_field_cols<F, VOLKOV> : k_field_cols<F, PHASE>;
     using RC = RCfg<F>;
     const size_t sm_vrows = RC::SMEM;
-    if (allow_smem(k_field_rows<F>, FC::SMEM) || allow_smem(k_field_cols<F>, CC::SMEM) ||
+    if (allow_smem(k_field_rows<F>, FC::SMEM) || allow_smem(field_cols, CC::SMEM) ||
         allow_smem(k_volkov_rows<L>, sm_vrows) || allow_smem(k_volkov_cols<L>, CC::SMEM) ||
         allow_smem(k_volkov_integ_rows<F>, IC::SMEM) || allow_smem(k_volkov_integ_cols<F>, CC::SMEM))
         return TDM_ECUDA;
@@ -640,9 +685,8 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
         }
         {
             Launch l(c, K_FIELD_COLS);
-            const bool keep = dbg_phase || !(p.deroul && p.volkov);
-            k_field_cols<F><<<dim3(F / CC::B, m), CC::NT, CC::SMEM, c->stream>>>(
-                b.I1, p.c_aber, b.tw, keep ? b.phase : nullptr, b.amp, b.zph, b.fields + (size_t)g0 * FF, b.phase_sum);
+            field_cols<<<dim3(F / CC::B, m), CC::NT, CC::SMEM, c->stream>>>(
+                b.I1, b.tw, b.phase, b.amp, b.zph, b.fields + (size_t)g0 * FF, b.phase_sum);
         }
         if (!p.c_aber) continue;
         const float* unw = b.phase;
@@ -666,7 +710,7 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
             {
                 Launch l(c, K_VOLKOV_INTEG_COLS);
                 k_volkov_integ_cols<F><<<dim3(F / 2 / CC::B, m), CC::NT, CC::SMEM, c->stream>>>(
-                    b.tq, b.phase_sum, F / CC::B, b.tw, reinterpret_cast<float2*>(b.unwrapped));
+                    b.tq, b.phase_sum, mean ? F / CC::B : 0, b.tw, reinterpret_cast<float2*>(b.unwrapped));
             }
             unw = b.unwrapped;
         }
@@ -677,8 +721,8 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
         }
         if (form) {
             Launch l(c, K_FORM);
-            k_form<<<dim3((unsigned)((FF + 255) / 256), m), 256, 0, c->stream>>>(unw, b.amp, b.beta, F, p.born,
-                                                                                b.fields + (size_t)g0 * FF);
+            k_form<<<dim3((F + kFormRows - 1) / kFormRows, m), 32 * kFormRows, 0, c->stream>>>(
+                unw, b.amp, b.beta, F, p.born, b.fields + (size_t)g0 * FF);
         }
         if (dbg_phase)
             cudaMemcpyAsync(dbg_phase + (g0 - a0) * FF, b.phase, m * FF * sizeof(float), cudaMemcpyDefault, c->stream);
@@ -708,8 +752,8 @@ void launch_aber_fit(tdm_ctx* c, const float* unw, int m) {
 void launch_form(tdm_ctx* c, const float* unw, int g0, int m) {
     const size_t FF = (size_t)c->p.F * c->p.F;
     Launch l(c, K_FORM);
-    k_form<<<dim3((unsigned)((FF + 255) / 256), m), 256, 0, c->stream>>>(unw, c->b.amp, c->b.beta, c->p.F, c->p.born,
-                                                                        c->b.fields + (size_t)g0 * FF);
+    k_form<<<dim3((c->p.F + kFormRows - 1) / kFormRows, m), 32 * kFormRows, 0, c->stream>>>(
+        unw, c->b.amp, c->b.beta, c->p.F, c->p.born, c->b.fields + (size_t)g0 * FF);
 }
 
 int launch_fields(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapped, float* dbg_amp, int argparts,
