@@ -178,19 +178,24 @@ k_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, cons
 // One warp per voxel column (X, Y).  An angle's cap window is the F x F bins
 // around its specular position, so a column is covered by a fraction of the
 // angles: a CTA first lists, in ascending order, the angles whose window covers
-// its row Y and any of its columns.  The lanes then take 32 consecutive listed
-// angles at a time: each lane loads its angle's cell plane in the column (a
-// 2-byte record), and the cap value only when the bin is a cap cell; the
-// planes of the next two groups and the values of the next group are loaded
-// while the current one is added, and groups without a hit are skipped.  An
-// angle hits a column at most once, at one plane, and the column's running
-// sums live in FP64 in shared memory.  When the group's planes are distinct
-// (seen through a plane -> lane ownership table) every lane adds its own hit;
-// otherwise lanes sharing a plane are grouped and the group's lowest lane sums
-// the members in ascending angle order (FP32, at most 32 terms) before adding
-// the sum.  The sums are deterministic, the hit counts exact.  Widening the
-// FP32 hits and narrowing the sums are done on the integer pipe (fp_bits.cuh),
-// so the FP64 pipe only adds.
+// its row Y and any of its columns, and takes them 32 at a time: its threads
+// load the 32 angles' cells of its columns (the plane, a 2-byte record, and the
+// cap value), neighbouring threads neighbouring columns, into a shared-memory
+// tile, the next 32 angles' cells on their way meanwhile, and a warp's lanes
+// then read its column's cells of the 32 angles.  (With the lanes loading their
+// angles' records themselves, every lane another line, the L1's data pipe was 85 %
+// busy and bounded the gather: 600 angles of 256^2 to 512^3 518 us.)  Groups
+// without a hit are skipped.  An angle hits a column at most once, at one plane.
+//
+// A column's running sums live in shared memory as pairs of floats: each hit is
+// added to the first by an error-free sum (Knuth's two-sum, on packed pairs of
+// real and imaginary part) whose error goes to the second, about 2^-48 of the
+// largest partial sum in all, where FP64 sums of FP32 group sums (the hits of 32
+// angles at one plane added in FP32 first) had that of an FP32 sum; FP64 adds run
+// at 1/64 of the FP32 rate here.  (Error of 600 random hits' sum, rounded to FP32:
+// 2.5e-8 relative, 3.2e-5 before; of positive hits 2.4e-8 and 2.5e-8.)  Hits of a group at the same plane are added
+// one after the other in ascending angle order, so the sums are deterministic;
+// the hit counts are exact.
 
 // A listed angle: its specular x and its index.  Both fit 16 bits: an angle is
 // listed only when its window meets the CTA's columns, which bounds x by the
@@ -248,154 +253,157 @@ __device__ __forceinline__ int list_angles(const int2* __restrict__ posspec, int
     return base;
 }
 
-// One warp sums column (bx, by) of the listed angles into acc (valid where cnt
-// is not 0) and cnt, band entries: the cells' planes and values are read from
-// the cap records at koff, the bin of the column in each angle's F x F window.
-__device__ __forceinline__ void gather_column(const float2* __restrict__ rec, const int16_t* __restrict__ recz,
-                                              const Listed* list, int listed, size_t FF, size_t koff, int bx, int F,
-                                              int zmin, int band, double2* acc, uint16_t* cnt, uint8_t* own,
-                                              float2* stg, int lane) {
-    for (int e = lane; e < (band + 1) / 2; e += 32) reinterpret_cast<uint32_t*>(cnt)[e] = 0;
-    // plane of listed angle i's cell in this column, or -1 when the angle's
-    // window misses the column or the bin is outside its cap; the cap
-    // value of a cell with plane z
-    auto fetch_z = [&](int i) {
-        int z = -1;
-        if (i < listed) {
-            const Listed q = list[i];
-            if ((unsigned)(bx + q.x) < (unsigned)F) z = __ldg(&recz[(size_t)q.angle * FF + koff]);
-        }
-        return z;
-    };
-    auto fetch_v = [&](int i, int z) {
-        return z >= 0 ? __ldg(&rec[(size_t)list[i].angle * FF + koff]) : make_float2(0.f, 0.f);
-    };
-    // adds v to cell e's sums (a cell's first hit starts them) and k to its count
-    auto add = [&](int e, float2 v, int k) {
-        const unsigned n = cnt[e];
-        double2 t = make_double2(0.0, 0.0);
-        if (n) t = acc[e];
-        t.x += widen(v.x);
-        t.y += widen(v.y);
-        acc[e] = t;
-        cnt[e] = (uint16_t)(n + k);
-    };
-    int z_nxt = fetch_z(lane), z_nxt2 = fetch_z(32 + lane);
-    float2 v_nxt = fetch_v(lane, z_nxt);
-    __syncwarp();
-    for (int g0 = 0; g0 < listed; g0 += 32) {
-        const int z = z_nxt;
-        const float2 r = v_nxt;
-        z_nxt = z_nxt2;
-        v_nxt = fetch_v(g0 + 32 + lane, z_nxt);
-        z_nxt2 = fetch_z(g0 + 64 + lane);
-        const int e = z >= 0 ? z - zmin : -1;
-        if (!__any_sync(0xffffffffu, e >= 0)) continue;
-        if (e >= 0) own[e] = (uint8_t)lane;
-        __syncwarp();
-        const bool shared_plane = e >= 0 && own[e] != lane;
-        if (!__any_sync(0xffffffffu, shared_plane)) {
-            if (e >= 0) add(e, r, 1);
+// A column's sums: acc (x, y: the sum; z, w: its error) is valid where cnt is not
+// 0; touched lists the `hit` cells with a hit.
+struct ColumnSums {
+    float4* acc;
+    uint16_t *cnt, *touched;
+    int hit;
+};
+
+// One warp adds 32 angles' cells of its column to the column's sums: this
+// lane's cell has plane z (or -1) and value v; lane l's value is vs[l * pitch].
+// The first lane at a plane adds the values of all lanes there.
+__device__ __forceinline__ void gather_add(ColumnSums& c, int z, float2 v, const float2* vs, int pitch, int zmin,
+                                           int lane) {
+    const int e = z >= 0 ? z - zmin : -1;
+    if (!__any_sync(0xffffffffu, e >= 0)) return;
+    const unsigned same = __match_any_sync(0xffffffffu, e), below = (1u << lane) - 1u;
+    const bool leads = e >= 0 && !(same & below);
+    const unsigned n = leads ? c.cnt[e] : 1;
+    const unsigned fresh = __ballot_sync(0xffffffffu, n == 0);
+    if (leads) {
+        float2 hi = v, lo = make_float2(0.f, 0.f);
+        auto add = [&](float2 u) {
+            const float2 s = c_add(hi, u), b = c_sub(s, hi);
+            lo = c_add(lo, c_add(c_sub(hi, c_sub(s, b)), c_sub(u, b)));
+            hi = s;
+        };
+        if (n) {
+            const float4 t = c.acc[e];
+            hi = make_float2(t.x, t.y), lo = make_float2(t.z, t.w);
+            add(v);
         } else {
-            const unsigned grp = __match_any_sync(0xffffffffu, e >= 0 ? e : -1 - lane);
-            stg[lane] = r;
-            __syncwarp();
-            if (e >= 0 && (grp & ((1u << lane) - 1)) == 0) {  // lowest lane of its plane group
-                float sx = 0.0f, sy = 0.0f;
-                for (unsigned g = grp; g; g &= g - 1) {
-                    const float2 u = stg[__ffs(g) - 1];
-                    sx += u.x;
-                    sy += u.y;
-                }
-                add(e, make_float2(sx, sy), __popc(grp));
-            }
+            c.touched[c.hit + __popc(fresh & below)] = (uint16_t)e;
         }
-        __syncwarp();
+        for (unsigned g = same & ~below & ~(1u << lane); g; g &= g - 1) add(vs[(__ffs(g) - 1) * pitch]);
+        c.acc[e] = make_float4(hi.x, hi.y, lo.x, lo.y);
+        c.cnt[e] = (uint16_t)(n + __popc(same));
     }
+    c.hit += __popc(fresh);
+    __syncwarp();
 }
 
-// k_gather: a CTA of kGW warps takes kGX consecutive columns at one Y, kGW at a
-// time, one per warp.  Each warp normalises its column's cells in place (not
-// normalised for the adjoint scatter; (-1)^(X+Y+Z) stands for the first
-// fftshift3D), and the CTA stores the kGW columns together as rows of
-// consecutive x (64-byte pieces) of the [e][y][x] spectrum, with the OTF mask
-// (Re != 0 after normalisation, main.cpp:262-267) and the counts, which one
-// column at a time would scatter plane by plane.  The grid covers the columns
-// that caps can reach; cells outside them and outside the band are cleared by
-// the host.
-//
-// Bound by issue and latency (FP64 sums in shared memory, dependent record
-// loads), so what counts is warps in flight: 4.2 KB of shared memory a warp at
-// a band of 220 planes.
-// 500 angles of 250^2, 512^3, all outputs: 528 us; with 16 columns' cells in a
-// tile beside the sums (72 KB a CTA) 575 us; the former kernel, which ran the z
-// transform too, 891 us.  64 angles of 512^2, 1024^3: 1.73, 3.66, 2.62 ms (the
-// empty blocks of 32 cells are skipped here).
-constexpr int kGW = 8, kGX = 16;
+// x / n, correctly rounded, from r the correctly rounded 1 / n (Markstein's
+// quotient correction); infinities and NaN as the division gives them.
+__device__ __forceinline__ float over(float x, float n, float r) {
+    const float q = x * r, rest = fmaf(-q, n, x);
+    return rest == rest ? fmaf(rest, r, q) : q;
+}
 
+// k_gather: a CTA of W warps takes W consecutive columns at one Y.  Each warp
+// normalises its column's cells in place (not normalised for the adjoint
+// scatter; (-1)^(X+Y+Z) stands for the first fftshift3D), and the CTA stores the
+// columns together as rows of consecutive x of the [e][y][x] spectrum, with the
+// OTF mask (Re != 0 after normalisation, main.cpp:262-267) and the counts, which
+// one column at a time would scatter plane by plane.  The grid covers the columns
+// that caps can reach; cells outside them and outside the band are cleared by
+// the host.  8 columns a CTA, for more warps an SM; with the counts of a volume
+// well beyond L2 16 columns, whose rows of counts are whole 64-byte pieces (300
+// angles of 256^2 to 512^3 418 -> 381 us, 64 of 512^2 to 1024^3 3.5 -> 2.3 ms; at
+// 256^3 8 columns take 76 us, 16 90).
+//
+// Bound by issue and latency.  600 angles of 256^2 to 512^3: 434 us (with FP64
+// sums of FP32 group sums, and each lane loading its angle's records, 538); 400
+// of 128^2 to 256^3 76 us (100).
+template <int W>
 struct GatherSmem {
-    // per warp: sums, counts (uint16), plane owners (uint8) and a 32-lane
-    // staging row, at a pitch of 16 bytes mod 128: with the normalised cell of
-    // an odd plane in the upper half of its sums' slot, the CTA-wide store's
-    // reads (8 columns x 2 planes a half-warp) fall in distinct banks
+    // per warp: sums, counts (uint16) and cells with a hit (uint16), at a pitch of
+    // 16 bytes mod 128: with the normalised cell of an odd plane in the upper half of its sums' slot, the
+    // CTA-wide store's reads fall in distinct banks.  Per CTA: two tiles of 32
+    // angles' cells (odd row pitches, so that a column is read without
+    // conflicts) and the list of angles.
+    static constexpr int VP = W + 1, ZP = W + 2;  // row pitches of a tile's values and planes
+    static constexpr int TILE = 32 * VP * 8 + 32 * ZP * 2;
     __host__ __device__ static int cnt_at(int band) { return band * 16; }
-    __host__ __device__ static int own_at(int band) { return cnt_at(band) + ((band * 2 + 15) & ~15); }
-    __host__ __device__ static int stg_at(int band) { return own_at(band) + ((band + 15) & ~15); }
-    __host__ __device__ static int pitch(int band) { return ((stg_at(band) + 32 * 8 - 16 + 127) & ~127) + 16; }
+    __host__ __device__ static int touched_at(int band) { return cnt_at(band) + ((band * 2 + 15) & ~15); }
+    __host__ __device__ static int pitch(int band) {
+        return ((touched_at(band) + ((band * 2 + 15) & ~15) - 16 + 127) & ~127) + 16;
+    }
     __host__ __device__ static size_t bytes(int band, int n) {
-        return (size_t)kGW * pitch(band) + (size_t)n * sizeof(Listed);
+        return (size_t)W * pitch(band) + 2 * TILE + (size_t)n * sizeof(Listed);
     }
 };
 
-__global__ void __launch_bounds__(kGW * 32)
+template <int W>
+__global__ void __launch_bounds__(W * 32, W == 8 ? 6 : 2)
 k_gather(const float2* __restrict__ rec, const int16_t* __restrict__ recz, const int2* __restrict__ posspec, int M,
          Params p, float2* __restrict__ vol, uint32_t* __restrict__ cnt_out, uint8_t* __restrict__ otf,
          int normalize) {
+    using S = GatherSmem<W>;
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ unsigned s_bal[2][32];
     const int band = p.band, F = p.F, D = p.D, h = D / 2, zmin = p.zmin;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int pitch = GatherSmem::pitch(band), cnt_at = GatherSmem::cnt_at(band);
+    const int pitch = S::pitch(band), cnt_at = S::cnt_at(band);
     unsigned char* mine = smraw + w * pitch;
-    double2* acc = reinterpret_cast<double2*>(mine);
-    uint16_t* cnt = reinterpret_cast<uint16_t*>(mine + cnt_at);
-    uint8_t* own = mine + GatherSmem::own_at(band);
-    float2* stg = reinterpret_cast<float2*>(mine + GatherSmem::stg_at(band));
-    Listed* list = reinterpret_cast<Listed*>(smraw + kGW * pitch);
-    auto cell = [](unsigned char* col, int e) { return reinterpret_cast<float2*>(col + e * 16 + (e & 1) * 8); };
+    ColumnSums col{reinterpret_cast<float4*>(mine), reinterpret_cast<uint16_t*>(mine + cnt_at),
+                   reinterpret_cast<uint16_t*>(mine + S::touched_at(band)), 0};
+    unsigned char* tile = smraw + W * pitch;
+    Listed* list = reinterpret_cast<Listed*>(tile + 2 * S::TILE);
+    auto cell = [](unsigned char* c, int e) { return reinterpret_cast<float2*>(c + e * 16 + (e & 1) * 8); };
     const size_t FF = (size_t)F * F, plane = (size_t)D * D;
-    const int X0 = p.xa + blockIdx.x * kGX, Y = p.ya + blockIdx.y, by = Y - h;
-    const int listed = list_angles<kGW>(posspec, M, F, by, X0 - h, kGX, list, s_bal);
-    const int ky = ((by % F) + F) % F;
-    for (int c0 = 0; c0 < kGX; c0 += kGW) {
-        const int X = X0 + c0 + w, bx = X - h;
-        gather_column(rec, recz, list, listed, FF, (size_t)ky * F + ((bx % F) + F) % F, bx, F, zmin, band, acc, cnt,
-                      own, stg, lane);
-        for (int e0 = 0; e0 < band; e0 += 32) {
-            const int e = e0 + lane;
-            const unsigned n = e < band ? cnt[e] : 0;
-            float2 v = make_float2(0.f, 0.f);
-            if (__any_sync(0xffffffffu, n != 0)) {
-                if (n) {
-                    const double2 t = acc[e];
-                    const float dn = normalize ? (float)n : 1.0f;  // FP32 division: FP64 division is a long sequence here
-                    v = make_float2(narrow(t.x) / dn, narrow(t.y) / dn);
-                }
-                if ((X + Y + zmin + e) & 1) v = make_float2(-v.x, -v.y);
+    const int X0 = p.xa + blockIdx.x * W, Y = p.ya + blockIdx.y, by = Y - h;
+    for (int e = lane; e < (band + 1) / 2; e += 32) reinterpret_cast<uint32_t*>(col.cnt)[e] = 0;
+    const int listed = list_angles<W>(posspec, M, F, by, X0 - h, W, list, s_bal);
+    // this thread's cell of a group of 32 listed angles: column c, angle i of the group
+    const int c = threadIdx.x % W, i = threadIdx.x / W, bx = X0 + c - h;
+    const size_t koff = (size_t)(((by % F) + F) % F) * F + ((bx % F) + F) % F;
+    float2 v = make_float2(0.f, 0.f);
+    int z = -1;
+    auto fetch = [&](int g0) {
+        z = -1;
+        if (g0 + i < listed) {
+            const Listed q = list[g0 + i];
+            if ((unsigned)(bx + q.x) < (unsigned)F) {  // the angle's window covers the column
+                const size_t o = (size_t)q.angle * FF + koff;
+                z = __ldg(&recz[o]);
+                v = __ldg(&rec[o]);
             }
-            if (e < band) *cell(mine, e) = v;
         }
-        __syncthreads();
-        const int c = threadIdx.x % kGW;
-        unsigned char* col = smraw + c * pitch;
-        size_t o = (size_t)Y * D + X0 + c0 + c + (threadIdx.x / kGW) * plane;
-        for (int e = threadIdx.x / kGW; e < band; e += 32, o += 32 * plane) {
-            const float2 v = *cell(col, e);
-            vol[o] = v;
-            if (cnt_out) cnt_out[zmin * plane + o] = reinterpret_cast<uint16_t*>(col + cnt_at)[e];
-            if (otf) otf[zmin * plane + o] = v.x != 0.0f;
+    };
+    fetch(0);
+    for (int g0 = 0, k = 0; g0 < listed; g0 += 32, k ^= 1) {
+        float2* tv = reinterpret_cast<float2*>(tile + k * S::TILE);
+        int16_t* tz = reinterpret_cast<int16_t*>(tv + 32 * S::VP);
+        tv[i * S::VP + c] = v;
+        tz[i * S::ZP + c] = (int16_t)z;
+        fetch(g0 + 32);
+        __syncthreads();  // the other tile is read before the barrier after this one
+        gather_add(col, tz[lane * S::ZP + w], tv[lane * S::VP + w], tv + w, S::VP, zmin, lane);
+    }
+    for (int t = lane; t < col.hit; t += 32) {
+        const int e = col.touched[t];
+        const float4 sum = col.acc[e];
+        float2 u = make_float2(sum.x + sum.z, sum.y + sum.w);
+        // an infinite sum has no error term
+        if (!(u.x == u.x)) u.x = sum.x;
+        if (!(u.y == u.y)) u.y = sum.y;
+        if (normalize) {
+            const float n = (float)col.cnt[e], r = __frcp_rn(n);
+            u = make_float2(over(u.x, n, r), over(u.y, n, r));
         }
-        if (c0 + kGW < kGX) __syncthreads();  // the next columns take the sums' place
+        *cell(mine, e) = ((X0 + w + Y + zmin + e) & 1) ? make_float2(-u.x, -u.y) : u;
+    }
+    __syncthreads();
+    unsigned char* from = smraw + c * pitch;
+    size_t o = (size_t)Y * D + X0 + c + i * plane;
+    for (int e = i; e < band; e += 32, o += 32 * plane) {
+        const unsigned n = reinterpret_cast<uint16_t*>(from + cnt_at)[e];
+        const float2 u = n ? *cell(from, e) : make_float2(0.f, 0.f);
+        vol[o] = u;
+        if (cnt_out) cnt_out[zmin * plane + o] = n;
+        if (otf) otf[zmin * plane + o] = u.x != 0.0f;
     }
 }
 
@@ -780,16 +788,23 @@ static cudaError_t download_after(tdm_ctx* c, cudaStream_t st, cudaEvent_t ev, v
 }
 
 // The gather of n angles' cap records into the band spectrum.
+template <int W>
+int launch_gather_as(tdm_ctx* c, CapRecs rec, const int2* posspec, int n, uint32_t* cnt, uint8_t* otf, int normalize,
+                     cudaStream_t st) {
+    const Params& p = c->p;
+    const size_t smem = GatherSmem<W>::bytes(p.band, n);
+    if (smem > kMaxSmemPerCta) return TDM_EUNSUPPORTED;
+    if (allow_smem(k_gather<W>, smem)) return TDM_ECUDA;
+    Launch l(c, K_GATHER, st);
+    k_gather<W><<<dim3((p.xb - p.xa) / W, p.yb - p.ya), W * 32, smem, st>>>(rec.val, rec.z, posspec, n, p, c->b.vol,
+                                                                            cnt, otf, normalize);
+    return TDM_OK;
+}
 int launch_gather(tdm_ctx* c, CapRecs rec, const int2* posspec, int n, uint32_t* cnt, uint8_t* otf, int normalize,
                   cudaStream_t st) {
-    const Params& p = c->p;
-    const size_t smem = GatherSmem::bytes(p.band, n);
-    if (smem > kMaxSmemPerCta) return TDM_EUNSUPPORTED;
-    if (allow_smem(k_gather, smem)) return TDM_ECUDA;
-    Launch l(c, K_GATHER, st);
-    k_gather<<<dim3((p.xb - p.xa) / kGX, p.yb - p.ya), kGW * 32, smem, st>>>(rec.val, rec.z, posspec, n, p, c->b.vol,
-                                                                             cnt, otf, normalize);
-    return TDM_OK;
+    if (cnt && c->p.D >= 512 && GatherSmem<16>::bytes(c->p.band, n) <= kMaxSmemPerCta)
+        return launch_gather_as<16>(c, rec, posspec, n, cnt, otf, normalize, st);
+    return launch_gather_as<8>(c, rec, posspec, n, cnt, otf, normalize, st);
 }
 
 // x and y passes on the band planes, after the gather (DIR +1).
