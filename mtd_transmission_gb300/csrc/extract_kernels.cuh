@@ -10,36 +10,34 @@
 namespace tdm {
 namespace extract {
 
-// Both passes run on the warp-resident FFT (fft_warp.cuh) in CTAs of 8
-// warps.  The row pass packs two real rows into one complex transform and
-// keeps the crop's kx band, written column-major (inter[a][c][y]): the two
-// rows' values of one column are one 16-byte word, and the CTA's row pairs
-// fill one segment of each column, stored whole from a shared-memory tile
-// (16-byte pieces of distinct lines, one per lane, would cost the L1 a
-// wavefront each and L2 a partial-sector write).  The column pass
-// then reads whole columns contiguously and writes the crop rows through a
-// shared-memory tile (and, on request, the crop's partial specular-peak
-// winners, one record per warp).
+// The row pass runs in CTAs of 8 warps, a warp per G row pairs: it packs two
+// real rows into one complex transform and keeps the crop's kx band, written row
+// by row (inter[a][y][c]).  The column pass's lanes run across columns (ColFFT):
+// it reads the band's rows, transforms the columns in registers and stores the
+// crop's rows, with the crop's partial specular-peak winners on request (one
+// record per warp), so that neither pass stages its data for the other's order.
+// Bound by issue (the row pass 63 % active at two CTAs an SM).  400 x 1024^2, F =
+// 256: rows 479 us with the band stored column by column through a tile, 397 like
+// this; columns 270 us as a warp per stored column with the crop through a tile,
+// 294 like this (64-byte pieces instead of whole columns, but 16 columns a CTA
+// leave one CTA an SM: 349); 64 x 2048^2 422 + 222 us, now 349 + 224.
 template <int H>
 struct ExtractCfg {
     using W = WarpFFT<H>;
-    static constexpr int NT = 256;         // threads per CTA
+    static constexpr int NT = 256;         // threads per CTA (rows pass)
     static constexpr int P = 8 * W::G;     // row pairs per CTA (rows pass)
-    static constexpr int C = 8 * W::G;     // columns per CTA (cols pass)
+    // columns per CTA: from 32 lanes a transform on 8, so that two CTAs (H =
+    // 1024) fit an SM's registers
+    using Cols = ColFFT<H, (W::T >= 32 ? 8 : 16)>;
     // row-pass CTAs per SM that the registers are capped for (shared memory
     // would allow 3 up to H = 1024, but capping to 80 registers for them
     // spills and measured slower than 2)
     static constexpr int ROWS_CTAS = H >= 2048 ? 1 : 2;
-    // band columns per round of the row pass's output tile (CB x (P + 1)
-    // 16-byte words, about 18 KB; the odd stride keeps both its column-wise
-    // fill and its row-wise drain free of bank conflicts)
-    static constexpr int CB = 1024 / P;
-    static size_t smem_rows(int) {
-        return (size_t)P * W::STRIDE * sizeof(float2) + (size_t)CB * (P + 1) * sizeof(float4);
-    }
-    static size_t smem_cols(int F) { return ((size_t)C * W::STRIDE + (size_t)F * (C + 1)) * sizeof(float2); }
+    static constexpr int COLS_CTAS = Cols::NT >= 512 || H >= 2048 ? 1 : 512 / Cols::NT;
+    static constexpr size_t SMEM_ROWS = (size_t)P * W::STRIDE * sizeof(float2);
     static dim3 grid_rows(int m) { return dim3(H / (2 * P), m); }
-    static dim3 grid_cols(int F, int m) { return dim3((F + C - 1) / C, m); }
+    static dim3 grid_cols(int F, int m) { return dim3((F + Cols::B - 1) / Cols::B, m); }
+    static int arg_parts(int F) { return (int)grid_cols(F, 1).x * (Cols::NT / 32); }
 };
 
 // Lanes' elements n1 whose pixels x = j + T n1 can fall in the hologram
@@ -147,77 +145,61 @@ k_extract_rows(const void* __restrict__ holos, int bits, const float2* __restric
     }
     __syncwarp();
     // separate the two real rows on the kx band: Xa = (Z(k) + conj Z(-k))/2, Xb = (Z(k) - conj Z(-k))/(2i),
-    // times the rows' window factors;
-    // rows ya (even) and yb = ya + 1 of column c are adjacent in inter (one
-    // 16-byte word), and the CTA's P row pairs are one 16P-byte segment of
-    // each column.  The words go through the tile, CB columns at a time, so
-    // that each column segment is written by consecutive lanes (whole lines)
-    // rather than as 16-byte pieces of distinct lines.
-    float4* tile = reinterpret_cast<float4*>(sm + P * W::STRIDE);
-    float4* dst = reinterpret_cast<float4*>(inter + (size_t)a * F * H + 2 * blockIdx.x * P);
-    for (int cb = 0; cb < F; cb += Cf::CB) {
-        const int nc = min(Cf::CB, F - cb);
-        for (int c = j; c < nc; c += T) {
-            const int k = x0 + cb + c, km = (H - k) & (H - 1);
-            const float2 z = s[W::pad(k)], zm = s[W::pad(km)];
-            tile[c * (P + 1) + tr] = make_float4(ha * (z.x + zm.x), ha * (z.y - zm.y), hb * (z.y + zm.y),
-                                                 -hb * (z.x - zm.x));
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < nc * P; i += Cf::NT) {
-            const int c = i / P, p = i % P;
-            dst[(size_t)(cb + c) * (H / 2) + p] = tile[c * (P + 1) + p];
-        }
-        if (cb + Cf::CB < F) __syncthreads();  // the tile is refilled
+    // times the rows' window factors
+    float2* dst = inter + ((size_t)a * H + ya) * F;
+#pragma unroll 4
+    for (int c = j; c < F; c += T) {
+        const int k = x0 + c, km = (H - k) & (H - 1);
+        const float2 z = s[W::pad(k)], zm = s[W::pad(km)];
+        dst[c] = make_float2(ha * (z.x + zm.x), ha * (z.y - zm.y));
+        dst[F + c] = make_float2(hb * (z.y + zm.y), -hb * (z.x - zm.x));
     }
 }
 
 template <int H>
-__global__ void __launch_bounds__(ExtractCfg<H>::NT)
+__global__ void __launch_bounds__(ExtractCfg<H>::Cols::NT, ExtractCfg<H>::COLS_CTAS)
 k_extract_cols(const float2* __restrict__ inter, const float2* __restrict__ tw, float2* __restrict__ spectra,
                int F, int x0, int y0, float4* __restrict__ argpart) {
-    using Cf = ExtractCfg<H>;
-    using W = typename Cf::W;
-    constexpr int T = W::T, E = W::E, C = Cf::C, TC = C + 1;
+    using C = typename ExtractCfg<H>::Cols;
+    using W = typename C::W;
+    constexpr int T = W::T, E = W::E;
     extern __shared__ __align__(16) float2 sm[];
-    float2* tile = sm + C * W::STRIDE;  // F x TC: [crop row][column in CTA]
-    const int tr = threadIdx.x / T, j = threadIdx.x % T;
-    const int a = blockIdx.y, c0 = blockIdx.x * C, c = c0 + tr;
-    const bool valid = c < F;  // the crop width need not be a multiple of C
-    float2* s = sm + tr * W::STRIDE;
-    const float2* src = inter + ((size_t)a * F + c) * H;
+    const int t = C::column(), j = C::adjacent_j();
+    const int a = blockIdx.y, c = blockIdx.x * C::B + t;
+    const bool valid = c < F;  // the crop width need not be a multiple of the columns
+    const float2* src = inter + (size_t)a * H * F + c;
     float2 x[E];
 #pragma unroll
-    for (int n1 = 0; n1 < E; ++n1) x[n1] = valid ? src[j + n1 * T] : make_float2(0.f, 0.f);
-    fft_warp_regs<H, -1>(x, s, j, tw);
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < E / T; ++q) {
-#pragma unroll
-        for (int k2 = 0; k2 < T; ++k2) s[warp_out_pos<H>(j, q, k2)] = x[q * T + k2];
-    }
-    __syncwarp();
-    const float inv = 1.0f / ((float)H * (float)H);
-    const int kx = x0 + c;
+    for (int n1 = 0; n1 < E; ++n1) x[n1] = valid ? src[(size_t)(j + n1 * T) * F] : make_float2(0.f, 0.f);
+    fft_cta_regs<H, -1>(x, sm + t * W::STRIDE, j, tw);
+    // (-1)^(kx+ky) / H^2: ky has j's parity
+    const float inv = 1.0f / ((float)H * (float)H), sg = ((x0 + c + j) & 1) ? -inv : inv;
+    float2* dst = spectra + (size_t)a * F * F + c;
     float best = -1.0f, second = -1.0f;
     int bi = 0x7fffffff;
-    for (int r = j; r < F; r += T) {
-        const int ky = y0 + r;
-        const float sg = ((kx + ky) & 1) ? -inv : inv;
-        const float2 z = c_scale(s[W::pad(ky)], sg);
-        tile[r * TC + tr] = z;
-        if (argpart && valid) argmax_take(best, bi, second, z, r * F + c);
+    dst += (ptrdiff_t)(j - y0) * F;
+    constexpr int GR = E >= 32 ? 4 : 2;  // output blocks of E rows tested for the crop together
+#pragma unroll
+    for (int g = 0; g < T / GR; ++g) {
+        if (E * GR * (g + 1) <= y0 || E * GR * g >= y0 + F) continue;
+#pragma unroll
+        for (int k = 0; k < GR; ++k) {
+#pragma unroll
+            for (int q = 0; q < E / T; ++q) {
+                const int k2 = g * GR + k, r = j + q * T + E * k2 - y0;  // crop row
+                if (valid && (unsigned)r < (unsigned)F) {
+                    const float2 z = c_scale(x[q * T + k2], sg);
+                    dst[(ptrdiff_t)(q * T + E * k2) * F] = z;
+                    if (argpart) argmax_take(best, bi, second, z, r * F + c);
+                }
+            }
+        }
     }
-    if (argpart) {  // this warp's partial winner of the specular search (8 records per CTA)
+    if (argpart) {  // this warp's partial winner of the specular search
         argmax_warp(best, bi, second);
         if ((threadIdx.x & 31) == 0)
-            argpart[((size_t)a * gridDim.x + blockIdx.x) * 8 + (threadIdx.x >> 5)] = argmax_record(best, bi, second);
-    }
-    __syncthreads();
-    float2* dst = spectra + (size_t)a * F * F + c0;
-    for (int i = threadIdx.x; i < F * C; i += Cf::NT) {
-        const int r = i / C, t = i % C;
-        if (c0 + t < F) dst[(size_t)r * F + t] = tile[r * TC + t];
+            argpart[((size_t)a * gridDim.x + blockIdx.x) * (C::NT / 32) + (threadIdx.x >> 5)] =
+                argmax_record(best, bi, second);
     }
 }
 

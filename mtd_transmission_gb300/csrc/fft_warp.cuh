@@ -232,15 +232,16 @@ __device__ __forceinline__ void fft_warp_regs(float2 (&x)[WarpFFT<N>::E], float2
 // times the traffic there).  A warp holds B = 16 columns of two lanes j: lane
 // pairs j and T - j (0 and T/2 in warp 0), so that bin N - k is held 16 lanes
 // away (in warp 0 by the lane itself), as the mirror passes want it.
-template <int N>
+template <int N, int COLS = 16>
 struct ColFFT {
     using W = WarpFFT<N>;
-    static constexpr int B = 16;
+    static constexpr int B = COLS;
     static constexpr int NT = B * W::T;
     static constexpr size_t SMEM = (size_t)B * W::STRIDE * sizeof(float2);
     __device__ static int column() { return threadIdx.x % B; }
     __device__ static int adjacent_j() { return threadIdx.x / B; }
-    __device__ static int paired_j() {
+    __device__ static int paired_j() {  // B = 16
+        static_assert(B == 16, "two lanes j a warp");
         const int w = threadIdx.x >> 5;
         return (threadIdx.x & 16) ? (w ? W::T - w : W::T / 2) : w;
     }

@@ -25,7 +25,7 @@ template <int H>
 int extract_impl(tdm_ctx* c, const void* holos, int bits, int n, int a0, bool argmax) {
     using C = ExtractCfg<H>;
     const Params& p = c->p;
-    const size_t sm_rows = C::smem_rows(p.F), sm_cols = C::smem_cols(p.F);
+    const size_t sm_rows = C::SMEM_ROWS, sm_cols = C::Cols::SMEM;
     if (!window_edge_ok(H, c->tuk_h_flat, win_edge<H>())) return TDM_EUNSUPPORTED;
     if (allow_smem(k_extract_rows<H, true>, sm_rows) != cudaSuccess) return TDM_ECUDA;
     if (allow_smem(k_extract_rows<H, false>, sm_rows) != cudaSuccess) return TDM_ECUDA;
@@ -46,13 +46,13 @@ int extract_impl(tdm_ctx* c, const void* holos, int bits, int n, int a0, bool ar
         }
         {
             Launch l(c, K_EXTRACT_COLS);
-            k_extract_cols<H><<<C::grid_cols(p.F, m), C::NT, sm_cols, c->stream>>>(
+            k_extract_cols<H><<<C::grid_cols(p.F, m), C::Cols::NT, sm_cols, c->stream>>>(
                 c->b.inter, c->b.tw, c->b.spectra + (size_t)(a0 + h0) * p.F * p.F, p.F, p.x0, p.y0,
                 argmax ? c->b.argpart : nullptr);
         }
     }
     if (cudaGetLastError() != cudaSuccess) return TDM_ECUDA;
-    return argmax ? (int)C::grid_cols(p.F, 1).x * (C::NT / 32) : TDM_OK;
+    return argmax ? C::arg_parts(p.F) : TDM_OK;
 }
 
 }  // namespace

@@ -58,7 +58,7 @@ struct Buffers {
     float2* s_pair = nullptr;      // the same values as pairs of floats (x the nearest float, x + y the value)
     float2* wq = nullptr;          // 4F, exp(-2 pi i k / 4F): twiddles of the mixed-radix passes
     uint8_t* holo_stage = nullptr; // host staging: 2 x chunk x H*H*2 bytes
-    float2* inter = nullptr;       // chunk x F x H (extraction row pass, kx band column-major)
+    float2* inter = nullptr;       // chunk x H x F (extraction row pass: the kx band, row-major)
     float2* spectra = nullptr;     // max_angles x F*F
     int2* posspec = nullptr;       // max_angles
     float2* specval = nullptr;     // max_angles

@@ -92,7 +92,7 @@ template <int H>
 int run(const Symbols& s, const void* holos, int bits, int n, float2* out, int F, int x0, int y0,
         cudaStream_t st) {
     using C = ExtractCfg<H>;
-    const size_t sm_rows = C::smem_rows(F), sm_cols = C::smem_cols(F);
+    const size_t sm_rows = C::SMEM_ROWS, sm_cols = C::Cols::SMEM;
     if (!window_edge_ok(H, tukey_flat(H, 0.05f), win_edge<H>())) return TDM_EUNSUPPORTED;
     if (sm_rows > 48 * 1024 &&
         cudaFuncSetAttribute(k_extract_rows<H, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_rows))
@@ -108,7 +108,7 @@ int run(const Symbols& s, const void* holos, int bits, int n, float2* out, int F
         k_extract_rows<H, false><<<C::grid_rows(m), C::NT, sm_rows, st>>>(
             static_cast<const char*>(holos) + h0 * in_bytes, bits, s.window + window_offset(H), nullptr, s.twiddle,
             s.scratch, F, x0, nullptr, 0u);
-        k_extract_cols<H><<<C::grid_cols(F, m), C::NT, sm_cols, st>>>(
+        k_extract_cols<H><<<C::grid_cols(F, m), C::Cols::NT, sm_cols, st>>>(
             s.scratch, s.twiddle, out + (size_t)h0 * F * F, F, x0, y0, nullptr);
     }
     return cudaGetLastError() == cudaSuccess ? TDM_OK : TDM_ECUDA;
