@@ -273,9 +273,11 @@ int tdm_set_wait_limit(tdm_ctx* ctx, long long polls);
  * streams the angles in chunks of `chunk` and keeps `lanes` consecutive chunks in
  * flight at once, each on its own stream with its own scratch (1 <= lanes <= 8,
  * chunk * lanes <= min(128, max_angles rounded up to a multiple of 16), the
- * scratch capacity of the context).  Default: 4 lanes and a quarter of the capacity
- * per chunk, less where the extracted bands of that many angles exceed the L2
- * cache, at least 16 (then fewer lanes if the capacity is smaller).  Waits for the context's queued work first.
+ * scratch capacity of the context).  Default, for holograms in host memory: 4
+ * lanes and a quarter of the capacity per chunk, less where the extracted bands
+ * of that many angles exceed the L2 cache, at least 16 (then fewer lanes if the
+ * capacity is smaller); in device memory: 2 lanes and half of the capacity, or 3
+ * lanes whose bands fit that cache.  Waits for the context's queued work first.
  * Results do not depend on the schedule. */
 int tdm_set_schedule(tdm_ctx* ctx, int chunk, int lanes);
 

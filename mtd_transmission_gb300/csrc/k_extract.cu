@@ -58,7 +58,7 @@ int extract_impl(tdm_ctx* c, const void* holos, int bits, int n, int a0, bool ar
 }  // namespace
 
 int launch_extract(tdm_ctx* c, const void* holos, int bits, int n, int a0, bool argmax) {
-    if (argmax && (n > c->holo_chunk || n > c->chunk)) return TDM_EINVAL;  // partials of one chunk only
+    if (argmax && n > c->chunk_cap) return TDM_EINVAL;  // partials of one chunk only
     switch (c->p.H) {
         case 256: return extract_impl<256>(c, holos, bits, n, a0, argmax);
         case 512: return extract_impl<512>(c, holos, bits, n, a0, argmax);

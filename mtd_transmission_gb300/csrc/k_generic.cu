@@ -529,7 +529,7 @@ int gcap_impl(tdm_ctx* c, int a0, int n, bool form) {
     if (allow_smem(gk_cap_rows<F, false>, sm_rows) || allow_smem(gk_cap_rows<F, true>, sm_rows) ||
         allow_smem(gk_cap_cols<F>, sm_cols))
         return TDM_ECUDA;
-    if (form && n > c->chunk) return TDM_EINVAL;  // the chunk buffers hold one chunk
+    if (form && n > c->chunk_cap) return TDM_EINVAL;  // the chunk buffers hold one chunk
     const size_t FF = (size_t)F * F;
     const unsigned rows = (F + kRows - 1) / kRows, cols = (F + kCols - 1) / kCols;
     const int step = angles_per_launch(c, n);

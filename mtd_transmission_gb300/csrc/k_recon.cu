@@ -752,7 +752,7 @@ int cap_impl(tdm_ctx* c, int a0, int n, bool form) {
     if (allow_smem(k_cap_rows<F>, C::SMEM) || allow_smem(k_cap_rows_form<F>, C::SMEM) ||
         allow_smem(k_cap_cols<F>, ColFFT<F>::SMEM))
         return TDM_ECUDA;
-    if (form && n > c->chunk) return TDM_EINVAL;  // the chunk buffers hold one chunk
+    if (form && n > c->chunk_cap) return TDM_EINVAL;  // the chunk buffers hold one chunk
     const size_t FF = (size_t)F * F;
     const int step = angles_per_launch(c, n);
     for (int g0 = a0; g0 < a0 + n; g0 += step) {

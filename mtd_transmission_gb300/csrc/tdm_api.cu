@@ -259,12 +259,21 @@ int tdm_create(const tdm_geom* geom, int max_angles, tdm_ctx** out) {
     p.rayon = c->dv.rayon;
     p.inv_rayon = 1.0 / c->dv.rayon;
     const int N = p.N, F = p.F, D = p.D;
-    // The pipeline's chunks: a quarter of the scratch each (200 x 512^2: (32, 4) 0.48, (16, 4) 0.65 ms a volume; 400
-    // x 256^2: 0.40, 0.64), but no more angles in flight than leave the extraction's band, the largest hand-over
-    // between two kernels, in L2 (600 x 1024^2, three contexts at once: (16, 4) 4.29, (32, 4) 4.42 ms), and no
-    // chunks of a few angles, whose launches cost more than they fill.
-    const int fit = (int)(kL2Bytes / ((size_t)p.H * F * sizeof(float2)));
-    c->chunk = c->holo_chunk = std::max(16, std::min(c->chunk_cap, fit) / c->lanes);
+    // The pipeline's chunks.  Holograms in host memory: four in flight, so that the uploads of later ones overlap, a
+    // quarter of the scratch each (200 x 512^2: (32, 4) 0.48, (16, 4) 0.65 ms a volume), but no more angles in flight
+    // than leave the extraction's band, the largest hand-over between two kernels, in L2, and no chunks of a few
+    // angles, whose launches cost more than they fill.
+    const size_t band_bytes = (size_t)p.H * F * sizeof(float2);
+    c->chunk = c->holo_chunk = std::max(16, std::min(c->chunk_cap, (int)(kL2Bytes / band_bytes)) / c->lanes);
+    // Holograms in device memory: fewer and larger launches, two chunks in flight, unless three chunks' bands can
+    // stay (nearly) in L2 where the whole scratch's cannot.  Volumes of one context alone / of three contexts in turn
+    // without waiting, in us: 600 x 1024^2 (16, 4) 3400/3770, (64, 2) 3230/3900, (24, 3) 3320/3450, (128, 1)
+    // 3550/3510; 64 x 2048^2 (16, 4) 8810/9100, (32, 2) 8810/8870; 200 x 512^2 (32, 4) 460/370, (64, 2) 450/360;
+    // 400 x 256^2 (32, 4) 430/300, (64, 2) 400/190.
+    const int three = (int)(kL2Bytes * 115 / 100 / (3 * band_bytes));
+    const bool keep = three >= 16 && (size_t)c->chunk_cap * band_bytes > kL2Bytes;
+    c->dev_lanes = keep ? 3 : 2;
+    c->dev_chunk = std::max(16, std::min(c->chunk_cap / c->dev_lanes, keep ? three : c->chunk_cap));
     // disc test fd^2 < COEF_NA_OBJ_LIMIT * N^2 on integers (fonctions.cpp:915)
     const double lim = geom->coef_na_obj_limit * (double)(N * N);
     p.disc_thr = (int)std::min<double>(std::ceil(lim), 2.0 * N * N + 1);
@@ -842,8 +851,9 @@ static int stage_angles(tdm_ctx* c, const void* holos, int bits, int n) {
     const Params& p = c->p;
     const size_t per = (size_t)p.H * p.H * (bits == 16 ? 2 : 1);
     const bool dev = is_device_ptr(holos);
-    const int nchunks = (n + c->holo_chunk - 1) / c->holo_chunk;
-    const int nl = std::max(1, std::min(std::min(c->lanes, kMaxLanes), std::min(c->chunk_cap / c->chunk, nchunks)));
+    const int chunk = dev ? c->dev_chunk : c->holo_chunk, lanes = dev ? c->dev_lanes : c->lanes;
+    const int nchunks = (n + chunk - 1) / chunk;
+    const int nl = std::max(1, std::min(std::min(lanes, kMaxLanes), std::min(c->chunk_cap / chunk, nchunks)));
     const int nslot = stage_slots(c), grp = upload_group(nslot);
     struct Restore {
         tdm_ctx* c;
@@ -855,13 +865,13 @@ static int stage_angles(tdm_ctx* c, const void* holos, int bits, int n) {
         }
     } restore{c, c->stream, scratch_at(c, 0)};
     ChunkScratch lane_scratch[kMaxLanes];
-    for (int l = 0; l < nl; ++l) lane_scratch[l] = scratch_at(c, l * c->chunk);
+    for (int l = 0; l < nl; ++l) lane_scratch[l] = scratch_at(c, l * chunk);
     if (nl > 1) {
         TDM_CU(cudaEventRecord(c->ev_lane_fork, restore.main));
         for (int l = 1; l < nl; ++l) TDM_CU(cudaStreamWaitEvent(c->lane_stream[l - 1], c->ev_lane_fork, 0));
     }
-    for (int h0 = 0, k = 0; h0 < n; h0 += c->holo_chunk, ++k) {
-        const int m = std::min(c->holo_chunk, n - h0);
+    for (int h0 = 0, k = 0; h0 < n; h0 += chunk, ++k) {
+        const int m = std::min(chunk, n - h0);
         const int lane = k % nl;
         c->stream = lane ? c->lane_stream[lane - 1] : restore.main;
         use_scratch(c, lane_scratch[lane]);
@@ -872,13 +882,13 @@ static int stage_angles(tdm_ctx* c, const void* holos, int bits, int n) {
             // go up in one copy, except that the call's first chunk goes alone
             // (its extraction starts after one chunk, not a group)
             const int ks = k < grp ? std::min(k, 1) : k - k % grp;
-            const size_t chunk_bytes = (size_t)c->holo_chunk * per;
+            const size_t chunk_bytes = (size_t)chunk * per;
             uint8_t* dst = stage_slot(c, buf0) + (size_t)(buf - buf0) * chunk_bytes;  // packed as on the host
             if (k == ks) {
                 const int cnt = std::min(k == 0 && grp > 1 ? 1 : grp - (k % grp), nchunks - k);
                 for (int q = 0; q < cnt; ++q)
                     TDM_CU(cudaStreamWaitEvent(c->copy_stream, c->ev_free[buf + q], 0));  // no-op before a first record
-                const size_t bytes = (size_t)std::min(cnt * c->holo_chunk, n - h0) * per;
+                const size_t bytes = (size_t)std::min(cnt * chunk, n - h0) * per;
                 TDM_CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->copy_stream));
                 TDM_CU(cudaEventRecord(c->ev_copy[buf], c->copy_stream));
             }
@@ -1186,8 +1196,8 @@ int tdm_set_schedule(tdm_ctx* c, int chunk, int lanes) {
         return fail(c, TDM_EINVAL, "tdm_set_schedule: need 1 <= lanes <= 8 and chunk * lanes <= the chunk capacity");
     cudaSetDevice(c->device);
     if (int rc = tdm_synchronize(c)) return rc;  // the staging ring's slots move with the chunk size
-    c->chunk = c->holo_chunk = chunk;
-    c->lanes = lanes;
+    c->chunk = c->holo_chunk = c->dev_chunk = chunk;
+    c->lanes = c->dev_lanes = lanes;
     return TDM_OK;
 }
 
@@ -1197,14 +1207,14 @@ int tdm_autotune(tdm_ctx* c, const void* holos, int bits, int n, int* chunk_out)
     cudaSetDevice(c->device);
     if (int rc = tdm_synchronize(c)) return rc;
     const int cands[][2] = {{16, 4}, {16, 2}, {8, 4}, {12, 4}, {32, 2}, {16, 6}, {32, 4}};
-    int best = c->chunk, best_lanes = c->lanes;
+    int best = c->dev_chunk, best_lanes = c->dev_lanes;
     float best_ms = 0;
     cudaEvent_t t0 = prof_event(c), t1 = prof_event(c);
     int rc = TDM_OK;
     for (const auto& cand : cands) {
         if (cand[0] * cand[1] > c->chunk_cap) continue;
-        c->chunk = c->holo_chunk = cand[0];
-        c->lanes = cand[1];
+        c->dev_chunk = cand[0];
+        c->dev_lanes = cand[1];
         rc = pipeline(c, holos, bits, n, nullptr, nullptr, nullptr, nullptr, nullptr, false);  // warm-up
         if (!rc && cudaEventRecord(t0, c->stream) != cudaSuccess) rc = TDM_ECUDA;
         for (int r = 0; r < 2 && !rc; ++r) rc = pipeline(c, holos, bits, n, nullptr, nullptr, nullptr, nullptr, nullptr, false);
@@ -1221,8 +1231,8 @@ int tdm_autotune(tdm_ctx* c, const void* holos, int bits, int n, int* chunk_out)
     }
     c->ev_pool.push_back(t0);
     c->ev_pool.push_back(t1);
-    c->chunk = c->holo_chunk = best;
-    c->lanes = best_lanes;
+    c->chunk = c->holo_chunk = c->dev_chunk = best;
+    c->lanes = c->dev_lanes = best_lanes;
     if (rc) return rc;
     if (chunk_out) *chunk_out = best;
     return TDM_OK;

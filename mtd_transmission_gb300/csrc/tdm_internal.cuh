@@ -123,6 +123,7 @@ struct tdm_ctx {
     int chunk = 16;              // angles per chunk of the pipeline's per-angle stages (tdm_set_schedule, tdm_autotune)
     int holo_chunk = 16;         // holograms per extraction chunk (equal to chunk)
     int lanes = 4;               // chunks in flight at once; lanes * chunk <= chunk_cap
+    int dev_chunk = 16, dev_lanes = 4;  // the same for holograms in device memory
     int chunk_cap = 64;          // angles of per-chunk scratch: min(128, max_angles rounded up to 16)
     int nsamp = 0;
     int device = 0;
