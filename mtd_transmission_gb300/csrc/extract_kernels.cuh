@@ -14,8 +14,8 @@ namespace extract {
 // real rows into one complex transform and keeps the crop's kx band, written row
 // by row (inter[a][y][c]).  The column pass's lanes run across columns (ColFFT):
 // it reads the band's rows, transforms the columns in registers and stores the
-// crop's rows, with the crop's partial specular-peak winners on request (one
-// record per warp), so that neither pass stages its data for the other's order.
+// crop's rows (to the caller's buffer as well, on request), with the crop's
+// partial specular-peak winners on request (one record per warp), so that neither pass stages its data for the other's order.
 // Bound by issue (the row pass 63 % active at two CTAs an SM).  400 x 1024^2, F =
 // 256: rows 479 us with the band stored column by column through a tile, 397 like
 // this; columns 270 us as a warp per stored column with the crop through a tile,
@@ -159,7 +159,7 @@ k_extract_rows(const void* __restrict__ holos, int bits, const float2* __restric
 template <int H>
 __global__ void __launch_bounds__(ExtractCfg<H>::Cols::NT, ExtractCfg<H>::COLS_CTAS)
 k_extract_cols(const float2* __restrict__ inter, const float2* __restrict__ tw, float2* __restrict__ spectra,
-               int F, int x0, int y0, float4* __restrict__ argpart) {
+               float2* __restrict__ also, int F, int x0, int y0, float4* __restrict__ argpart) {
     using C = typename ExtractCfg<H>::Cols;
     using W = typename C::W;
     constexpr int T = W::T, E = W::E;
@@ -190,6 +190,7 @@ k_extract_cols(const float2* __restrict__ inter, const float2* __restrict__ tw, 
                 if (valid && (unsigned)r < (unsigned)F) {
                     const float2 z = c_scale(x[q * T + k2], sg);
                     dst[(ptrdiff_t)(q * T + E * k2) * F] = z;
+                    if (also) also[(size_t)a * F * F + (size_t)r * F + c] = z;
                     if (argpart) argmax_take(best, bi, second, z, r * F + c);
                 }
             }

@@ -22,7 +22,7 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
 }
 
 template <int H>
-int extract_impl(tdm_ctx* c, const void* holos, int bits, int n, int a0, bool argmax) {
+int extract_impl(tdm_ctx* c, const void* holos, int bits, int n, int a0, bool argmax, float2* also) {
     using C = ExtractCfg<H>;
     const Params& p = c->p;
     const size_t sm_rows = C::SMEM_ROWS, sm_cols = C::Cols::SMEM;
@@ -47,7 +47,8 @@ int extract_impl(tdm_ctx* c, const void* holos, int bits, int n, int a0, bool ar
         {
             Launch l(c, K_EXTRACT_COLS);
             k_extract_cols<H><<<C::grid_cols(p.F, m), C::Cols::NT, sm_cols, c->stream>>>(
-                c->b.inter, c->b.tw, c->b.spectra + (size_t)(a0 + h0) * p.F * p.F, p.F, p.x0, p.y0,
+                c->b.inter, c->b.tw, c->b.spectra + (size_t)(a0 + h0) * p.F * p.F,
+                also ? also + (size_t)h0 * p.F * p.F : nullptr, p.F, p.x0, p.y0,
                 argmax ? c->b.argpart : nullptr);
         }
     }
@@ -57,13 +58,13 @@ int extract_impl(tdm_ctx* c, const void* holos, int bits, int n, int a0, bool ar
 
 }  // namespace
 
-int launch_extract(tdm_ctx* c, const void* holos, int bits, int n, int a0, bool argmax) {
+int launch_extract(tdm_ctx* c, const void* holos, int bits, int n, int a0, bool argmax, float2* also) {
     if (argmax && n > c->chunk_cap) return TDM_EINVAL;  // partials of one chunk only
     switch (c->p.H) {
-        case 256: return extract_impl<256>(c, holos, bits, n, a0, argmax);
-        case 512: return extract_impl<512>(c, holos, bits, n, a0, argmax);
-        case 1024: return extract_impl<1024>(c, holos, bits, n, a0, argmax);
-        case 2048: return extract_impl<2048>(c, holos, bits, n, a0, argmax);
+        case 256: return extract_impl<256>(c, holos, bits, n, a0, argmax, also);
+        case 512: return extract_impl<512>(c, holos, bits, n, a0, argmax, also);
+        case 1024: return extract_impl<1024>(c, holos, bits, n, a0, argmax, also);
+        case 2048: return extract_impl<2048>(c, holos, bits, n, a0, argmax, also);
         default: return TDM_EUNSUPPORTED;
     }
 }

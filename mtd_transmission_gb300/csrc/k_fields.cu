@@ -52,14 +52,20 @@ cudaError_t allow_smem(K kernel, size_t bytes) {
 // of each spectrum (k_argmax_part here, or the extraction column pass when
 // the spectra come straight from the holograms), then argmax_final in
 // k_field_rows, the first consumer.
+// copy (may be null) receives the spectra.
 __global__ void __launch_bounds__(256) k_argmax_part(const float2* __restrict__ spectra, int F,
-                                                     float4* __restrict__ part) {
+                                                     float4* __restrict__ part, float2* __restrict__ copy) {
     const int a = blockIdx.y, sl = blockIdx.x;
     const int per = (F * F + kArgSlices - 1) / kArgSlices, i0 = sl * per, i1 = min(i0 + per, F * F);
     const float2* s = spectra + (size_t)a * F * F;
     float best = -1.0f, second = -1.0f;
     int bi = 0x7fffffff;
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) argmax_take(best, bi, second, s[i], i);
+#pragma unroll 4
+    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+        const float2 z = s[i];
+        if (copy) copy[(size_t)a * F * F + i] = z;
+        argmax_take(best, bi, second, z, i);
+    }
     argmax_block(best, bi, second);
     if (threadIdx.x == 0) part[(size_t)a * kArgSlices + sl] = argmax_record(best, bi, second);
 }
@@ -635,7 +641,7 @@ __global__ void __launch_bounds__(kFitThreads) k_aber_fit(const float* __restric
 constexpr int kFormRows = 8;  // rows (warps) per CTA
 __global__ void __launch_bounds__(32 * kFormRows)
 k_form(const float* __restrict__ unwrapped, const float* __restrict__ amp, const double* __restrict__ beta, int F,
-       int born, float2* __restrict__ fields) {
+       int born, float2* __restrict__ fields, float2* __restrict__ also) {
     const int a = blockIdx.y, y = blockIdx.x * kFormRows + (threadIdx.x >> 5);
     __shared__ float bf[2 * kNC];
     if (threadIdx.x < 2 * kNC) bf[threadIdx.x] = (float)beta[(size_t)a * 2 * kNC + threadIdx.x];
@@ -644,13 +650,16 @@ k_form(const float* __restrict__ unwrapped, const float* __restrict__ amp, const
     const FormRow r = form_row(bf, y, F);
     const size_t row = ((size_t)a * F + y) * F;
 #pragma unroll 4
-    for (int x = threadIdx.x & 31; x < F; x += 32)
-        fields[row + x] = form_value(r, x, F, unwrapped[row + x], amp[row + x], born);
+    for (int x = threadIdx.x & 31; x < F; x += 32) {
+        const float2 f = form_value(r, x, F, unwrapped[row + x], amp[row + x], born);
+        fields[row + x] = f;
+        if (also) also[row + x] = f;
+    }
 }
 
 template <int F>
 int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapped, float* dbg_amp, int argparts,
-                bool form) {
+                bool form, FieldIo io) {
     constexpr int L = 2 * F;
     using FC = FieldCfg<F>;
     using CC = ColFFT<F>;
@@ -671,13 +680,9 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
     const int step = angles_per_launch(c, n);
     for (int g0 = a0; g0 < a0 + n; g0 += step) {
         const int m = a0 + n - g0 < step ? a0 + n - g0 : step;
-        const float2* spec = b.spectra + (size_t)g0 * FF;
-        int nparts = argparts;
-        if (!nparts) {
-            Launch l(c, K_ARGMAX);
-            k_argmax_part<<<dim3(kArgSlices, m), 256, 0, c->stream>>>(spec, F, b.argpart);
-            nparts = kArgSlices;
-        }
+        float2* spec = b.spectra + (size_t)g0 * FF;
+        const float2* in = io.spectra ? io.spectra + (size_t)(g0 - a0) * FF : spec;
+        const int nparts = argparts ? argparts : launch_argmax_part(c, in, m, io.spectra ? spec : nullptr);
         {
             Launch l(c, K_FIELD_ROWS);
             k_field_rows<F><<<dim3(F / FC::B, m), FC::NT, FC::SMEM, c->stream>>>(
@@ -714,16 +719,8 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
             }
             unw = b.unwrapped;
         }
-        {
-            Launch l(c, K_ABER_FIT);
-            k_aber_fit<<<dim3(kFitSlices, 2, m), kFitThreads, 0, c->stream>>>(
-                unw, b.amp, b.samp_idx, b.samp_q, c->nsamp, F, b.rinv, b.fit_part, b.fit_done, b.beta);
-        }
-        if (form) {
-            Launch l(c, K_FORM);
-            k_form<<<dim3((F + kFormRows - 1) / kFormRows, m), 32 * kFormRows, 0, c->stream>>>(
-                unw, b.amp, b.beta, F, p.born, b.fields + (size_t)g0 * FF);
-        }
+        launch_aber_fit(c, unw, m);
+        if (form) launch_form(c, unw, g0, m, io.fields ? io.fields + (size_t)(g0 - a0) * FF : nullptr);
         if (dbg_phase)
             cudaMemcpyAsync(dbg_phase + (g0 - a0) * FF, b.phase, m * FF * sizeof(float), cudaMemcpyDefault, c->stream);
         if (dbg_unwrapped)
@@ -736,9 +733,9 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
 
 }  // namespace
 
-int launch_argmax_part(tdm_ctx* c, const float2* spec, int m) {
+int launch_argmax_part(tdm_ctx* c, const float2* spec, int m, float2* copy) {
     Launch l(c, K_ARGMAX);
-    k_argmax_part<<<dim3(kArgSlices, m), 256, 0, c->stream>>>(spec, c->p.F, c->b.argpart);
+    k_argmax_part<<<dim3(kArgSlices, m), 256, 0, c->stream>>>(spec, c->p.F, c->b.argpart, copy);
     return kArgSlices;
 }
 
@@ -749,21 +746,22 @@ void launch_aber_fit(tdm_ctx* c, const float* unw, int m) {
                                                                       c->b.fit_done, c->b.beta);
 }
 
-void launch_form(tdm_ctx* c, const float* unw, int g0, int m) {
+void launch_form(tdm_ctx* c, const float* unw, int g0, int m, float2* also) {
     const size_t FF = (size_t)c->p.F * c->p.F;
     Launch l(c, K_FORM);
     k_form<<<dim3((c->p.F + kFormRows - 1) / kFormRows, m), 32 * kFormRows, 0, c->stream>>>(
-        unw, c->b.amp, c->b.beta, c->p.F, c->p.born, c->b.fields + (size_t)g0 * FF);
+        unw, c->b.amp, c->b.beta, c->p.F, c->p.born, c->b.fields + (size_t)g0 * FF, also);
 }
 
 int launch_fields(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapped, float* dbg_amp, int argparts,
-                  bool form) {
-    if (c->p.F & (c->p.F - 1)) return launch_fields_generic(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form);
+                  bool form, FieldIo io) {
+    if (c->p.F & (c->p.F - 1))
+        return launch_fields_generic(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form, io);
     switch (c->p.F) {
-        case 64: return fields_impl<64>(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form);
-        case 128: return fields_impl<128>(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form);
-        case 256: return fields_impl<256>(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form);
-        case 512: return fields_impl<512>(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form);
+        case 64: return fields_impl<64>(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form, io);
+        case 128: return fields_impl<128>(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form, io);
+        case 256: return fields_impl<256>(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form, io);
+        case 512: return fields_impl<512>(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form, io);
         default: return TDM_EUNSUPPORTED;
     }
 }

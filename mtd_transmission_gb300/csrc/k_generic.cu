@@ -400,6 +400,7 @@ gk_cap_rows(const float2* __restrict__ fields_in, const float* __restrict__ unwr
             fields_out[row + x] = f;
         } else {
             f = fields_in[row + x];
+            if (fields_out) fields_out[row + x] = f;
         }
         A[x] = c_scale(f, ((x >= flat.x && x <= flat.y) ? 1.0f : __ldg(&tuk[x])) * wy);
     }
@@ -454,7 +455,7 @@ constexpr size_t warp_arrays(int n, int warps) { return (size_t)warps * 2 * n * 
 
 template <int F>
 int gfields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapped, float* dbg_amp, int argparts,
-                 bool form) {
+                 bool form, FieldIo io) {
     const Params& p = c->p;
     Buffers& b = c->b;
     const size_t FF = (size_t)F * F;
@@ -470,8 +471,9 @@ int gfields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapp
     const int step = angles_per_launch(c, n);
     for (int g0 = a0; g0 < a0 + n; g0 += step) {
         const int m = a0 + n - g0 < step ? a0 + n - g0 : step;
-        const float2* spec = b.spectra + (size_t)g0 * FF;
-        const int nparts = argparts ? argparts : launch_argmax_part(c, spec, m);
+        float2* spec = b.spectra + (size_t)g0 * FF;
+        const float2* in = io.spectra ? io.spectra + (size_t)(g0 - a0) * FF : spec;
+        const int nparts = argparts ? argparts : launch_argmax_part(c, in, m, io.spectra ? spec : nullptr);
         {
             Launch l(c, K_FIELD_ROWS);
             gk_field_rows<F><<<dim3(rows, m), kRows * 32, sm_rows, c->stream>>>(
@@ -511,7 +513,7 @@ int gfields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapp
             unw = b.unwrapped;
         }
         launch_aber_fit(c, unw, m);
-        if (form) launch_form(c, unw, g0, m);
+        if (form) launch_form(c, unw, g0, m, io.fields ? io.fields + (size_t)(g0 - a0) * FF : nullptr);
         if (dbg_phase)
             cudaMemcpyAsync(dbg_phase + (g0 - a0) * FF, b.phase, m * FF * sizeof(float), cudaMemcpyDefault, c->stream);
         if (dbg_unwrapped)
@@ -523,7 +525,7 @@ int gfields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapp
 }
 
 template <int F>
-int gcap_impl(tdm_ctx* c, int a0, int n, bool form) {
+int gcap_impl(tdm_ctx* c, int a0, int n, bool form, const float2* fields_in) {
     Buffers& b = c->b;
     const size_t sm_rows = warp_arrays(F, kRows), sm_cols = warp_arrays(F, kCols);
     if (allow_smem(gk_cap_rows<F, false>, sm_rows) || allow_smem(gk_cap_rows<F, true>, sm_rows) ||
@@ -543,7 +545,8 @@ int gcap_impl(tdm_ctx* c, int a0, int n, bool form) {
                     b.wq, b.fields + g0 * FF, b.r1);
             else
                 gk_cap_rows<F, false><<<dim3(rows, m), kRows * 32, sm_rows, c->stream>>>(
-                    b.fields + g0 * FF, nullptr, nullptr, nullptr, 0, b.tuk_f, c->tuk_f_flat, b.wq, nullptr, b.r1);
+                    fields_in ? fields_in + (g0 - a0) * FF : b.fields + g0 * FF, nullptr, nullptr, nullptr, 0, b.tuk_f,
+                    c->tuk_f_flat, b.wq, fields_in ? b.fields + g0 * FF : nullptr, b.r1);
         }
         {
             Launch l(c, K_CAP_COLS);
@@ -562,16 +565,16 @@ int gcap_impl(tdm_ctx* c, int a0, int n, bool form) {
 bool generic_field_size(int F) { return F == 250; }
 
 int launch_fields_generic(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapped, float* dbg_amp,
-                          int argparts, bool form) {
+                          int argparts, bool form, FieldIo io) {
     switch (c->p.F) {
-        case 250: return gfields_impl<250>(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form);
+        case 250: return gfields_impl<250>(c, a0, n, dbg_phase, dbg_unwrapped, dbg_amp, argparts, form, io);
         default: return TDM_EUNSUPPORTED;
     }
 }
 
-int launch_cap_generic(tdm_ctx* c, int a0, int n, bool form) {
+int launch_cap_generic(tdm_ctx* c, int a0, int n, bool form, const float2* fields_in) {
     switch (c->p.F) {
-        case 250: return gcap_impl<250>(c, a0, n, form);
+        case 250: return gcap_impl<250>(c, a0, n, form, fields_in);
         default: return TDM_EUNSUPPORTED;
     }
 }

@@ -47,10 +47,11 @@ struct CapCfg {
     static constexpr size_t SMEM = (size_t)B * W::STRIDE * sizeof(float2);
 };
 
+// copy (may be null) receives the fields.
 template <int F>
 __global__ void __launch_bounds__(CapCfg<F>::NT)
 k_cap_rows(const float2* __restrict__ fields, const float* __restrict__ tuk, int2 flat, const float2* __restrict__ tw,
-           float2* __restrict__ r1) {
+           float2* __restrict__ r1, float2* __restrict__ copy) {
     using C = CapCfg<F>;
     using W = typename C::W;
     constexpr int T = W::T, E = W::E;
@@ -63,7 +64,16 @@ k_cap_rows(const float2* __restrict__ fields, const float* __restrict__ tuk, int
 #pragma unroll
     for (int n1 = 0; n1 < E; ++n1) {
         const int xx = j + n1 * T;
-        x[n1] = c_scale(src[xx], ((xx >= flat.x && xx <= flat.y) ? 1.0f : __ldg(&tuk[xx])) * wy);
+        x[n1] = src[xx];
+    }
+    if (copy) {
+#pragma unroll
+        for (int n1 = 0; n1 < E; ++n1) copy[((size_t)a * F + y) * F + j + n1 * T] = x[n1];
+    }
+#pragma unroll
+    for (int n1 = 0; n1 < E; ++n1) {
+        const int xx = j + n1 * T;
+        x[n1] = c_scale(x[n1], ((xx >= flat.x && xx <= flat.y) ? 1.0f : __ldg(&tuk[xx])) * wy);
     }
     fft_warp_regs<F, -1>(x, sm + tr * W::STRIDE, j, tw);
     float2* dst = r1 + ((size_t)a * F + y) * F;
@@ -746,7 +756,7 @@ k_tv_step(TvChannel c0, TvChannel c1, int log_d, float step, float eps2) {
 }
 
 template <int F>
-int cap_impl(tdm_ctx* c, int a0, int n, bool form) {
+int cap_impl(tdm_ctx* c, int a0, int n, bool form, const float2* fields_in) {
     using C = CapCfg<F>;
     Buffers& b = c->b;
     if (allow_smem(k_cap_rows<F>, C::SMEM) || allow_smem(k_cap_rows_form<F>, C::SMEM) ||
@@ -764,8 +774,9 @@ int cap_impl(tdm_ctx* c, int a0, int n, bool form) {
                 b.fields + g0 * FF, b.r1);
         } else {
             Launch l(c, K_CAP_ROWS);
-            k_cap_rows<F><<<dim3(F / C::B, m), C::NT, C::SMEM, c->stream>>>(b.fields + g0 * FF, b.tuk_f,
-                                                                             c->tuk_f_flat, b.tw, b.r1);
+            k_cap_rows<F><<<dim3(F / C::B, m), C::NT, C::SMEM, c->stream>>>(
+                fields_in ? fields_in + (g0 - a0) * FF : b.fields + g0 * FF, b.tuk_f, c->tuk_f_flat, b.tw, b.r1,
+                fields_in ? b.fields + g0 * FF : nullptr);
         }
         {
             Launch l(c, K_CAP_COLS);
@@ -957,13 +968,13 @@ size_t gather_limit_bytes(int D, int band, int n) {
     return 4 * (region + 32 * sizeof(float2) + ((band + 15) & ~15)) + (((size_t)band * 4 + 7) & ~size_t(7)) +
            (size_t)n * sizeof(int2);
 }
-int launch_cap(tdm_ctx* c, int a0, int n, bool form) {
-    if (c->p.F & (c->p.F - 1)) return launch_cap_generic(c, a0, n, form);
+int launch_cap(tdm_ctx* c, int a0, int n, bool form, const float2* fields_in) {
+    if (c->p.F & (c->p.F - 1)) return launch_cap_generic(c, a0, n, form, fields_in);
     switch (c->p.F) {
-        case 64: return cap_impl<64>(c, a0, n, form);
-        case 128: return cap_impl<128>(c, a0, n, form);
-        case 256: return cap_impl<256>(c, a0, n, form);
-        case 512: return cap_impl<512>(c, a0, n, form);
+        case 64: return cap_impl<64>(c, a0, n, form, fields_in);
+        case 128: return cap_impl<128>(c, a0, n, form, fields_in);
+        case 256: return cap_impl<256>(c, a0, n, form, fields_in);
+        case 512: return cap_impl<512>(c, a0, n, form, fields_in);
         default: return TDM_EUNSUPPORTED;
     }
 }

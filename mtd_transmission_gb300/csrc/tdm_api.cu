@@ -86,6 +86,25 @@ bool is_device_ptr(const void* p) {
     return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
+// A caller's complex buffer that kernels may read or write themselves: memory of
+// the context's GPU, on an 8-byte boundary.  Others are copied.
+bool is_direct(const tdm_ctx* c, const void* p) {
+    cudaPointerAttributes at;
+    if (!p || (reinterpret_cast<uintptr_t>(p) & 7)) return false;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == c->device);
+}
+
+// Kernels write a caller's output while other chunks of its input are unread, so
+// buffers that share memory go through copies.
+bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + nb && y < x + na;
+}
+
 template <class T>
 int dev_alloc(tdm_ctx* c, T** p, size_t count) {
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(T));
@@ -650,10 +669,10 @@ static int upload_group(int nslot) {
     return 1;
 }
 
-static int stage_extract(tdm_ctx* c, const void* holos, int bits, int n) {
+static int stage_extract(tdm_ctx* c, const void* holos, int bits, int n, float2* also) {
     const Params& p = c->p;
     const size_t per = (size_t)p.H * p.H * (bits == 16 ? 2 : 1);
-    if (is_device_ptr(holos)) return launch_extract(c, holos, bits, n, 0);
+    if (is_device_ptr(holos)) return launch_extract(c, holos, bits, n, 0, false, also);
     // host holograms: chunked copies on the copy stream into a ring of staging slots
     const int nslot = stage_slots(c);
     for (int h0 = 0, k = 0; h0 < n; h0 += c->holo_chunk, ++k) {
@@ -665,7 +684,7 @@ static int stage_extract(tdm_ctx* c, const void* holos, int bits, int n) {
                                c->copy_stream));
         TDM_CU(cudaEventRecord(c->ev_copy[buf], c->copy_stream));
         TDM_CU(cudaStreamWaitEvent(c->stream, c->ev_copy[buf], 0));
-        if (int rc = launch_extract(c, dst, bits, m, h0)) return rc;
+        if (int rc = launch_extract(c, dst, bits, m, h0, false, also ? also + (size_t)h0 * p.F * p.F : nullptr)) return rc;
         TDM_CU(cudaEventRecord(c->ev_free[buf], c->stream));
     }
     return TDM_OK;
@@ -677,11 +696,14 @@ int tdm_extract(tdm_ctx* c, const void* holos, int bits, int n, float* spectra_o
     cudaSetDevice(c->device);
     TDM_CU(join_volume(c));
     TDM_CU(cudaEventRecord(c->ev_stage[0], c->stream));
-    if (int rc = stage_extract(c, holos, bits, n)) return rc;
+    const size_t FF = (size_t)c->p.F * c->p.F;
+    const bool direct = is_direct(c, spectra_out) &&
+                        !overlap(holos, (size_t)n * c->p.H * c->p.H * (bits / 8), spectra_out, n * FF * sizeof(float2));
+    float2* also = direct ? reinterpret_cast<float2*>(spectra_out) : nullptr;
+    if (int rc = stage_extract(c, holos, bits, n, also)) return rc;
     TDM_CU(cudaEventRecord(c->ev_stage[1], c->stream));
     c->n_spectra = n;
-    const size_t FF = (size_t)c->p.F * c->p.F;
-    if (spectra_out)
+    if (spectra_out && !also)
         TDM_CU(cudaMemcpyAsync(spectra_out, c->b.spectra, n * FF * sizeof(float2), cudaMemcpyDefault, c->stream));
     if (!is_device_ptr(holos) || (spectra_out && !is_device_ptr(spectra_out))) return tdm_synchronize(c);
     return TDM_OK;
@@ -693,17 +715,22 @@ static int run_fields(tdm_ctx* c, const float* spectra_in, int n, float* fields_
     cudaSetDevice(c->device);
     TDM_CU(join_volume(c));
     const size_t FF = (size_t)c->p.F * c->p.F;
-    if (spectra_in && spectra_in != reinterpret_cast<float*>(c->b.spectra)) {
+    FieldIo io;
+    if (c->p.c_aber && is_direct(c, fields_out)) io.fields = reinterpret_cast<float2*>(fields_out);
+    if (is_direct(c, spectra_in) &&
+        !(io.fields && overlap(spectra_in, n * FF * sizeof(float2), fields_out, n * FF * sizeof(float2))))
+        io.spectra = reinterpret_cast<const float2*>(spectra_in);
+    if (spectra_in && !io.spectra && spectra_in != reinterpret_cast<float*>(c->b.spectra)) {
         TDM_CU(cudaMemcpyAsync(c->b.spectra, spectra_in, n * FF * sizeof(float2), cudaMemcpyDefault, c->stream));
     } else if (!spectra_in && n > c->n_spectra) {
         return fail(c, TDM_EINVAL, "tdm_fields: fewer spectra in the context than requested");
     }
     TDM_CU(cudaEventRecord(c->ev_stage[1], c->stream));
-    if (int rc = launch_fields(c, 0, n, dph, dun, dam)) return fail(c, rc, "tdm_fields: kernel launch failed");
+    if (int rc = launch_fields(c, 0, n, dph, dun, dam, 0, true, io)) return fail(c, rc, "tdm_fields: kernel launch failed");
     TDM_CU(cudaEventRecord(c->ev_stage[2], c->stream));
     c->n_fields = n;
     bool host = (spectra_in && !is_device_ptr(spectra_in));
-    if (fields_out) {
+    if (fields_out && !io.fields) {
         TDM_CU(cudaMemcpyAsync(fields_out, c->b.fields, n * FF * sizeof(float2), cudaMemcpyDefault, c->stream));
         host |= !is_device_ptr(fields_out);
     }
@@ -739,10 +766,11 @@ int tdm_fields_debug(tdm_ctx* c, const float* spectra_in, int n, float* fields_o
 // device staging buffers and downloaded while the later passes run.
 static int run_volume(tdm_ctx* c, int n, bool cap, float* re, float* im, uint8_t* otf, uint32_t* cnt,
                       bool wait = true, cudaStream_t st = nullptr, const CapRecs* rec = nullptr,
-                      const int2* posspec = nullptr, cudaEvent_t ev_gathered = nullptr) {
+                      const int2* posspec = nullptr, cudaEvent_t ev_gathered = nullptr,
+                      const float2* fields_in = nullptr) {
     const Params& p = c->p;
     const size_t NT = (size_t)p.D * p.D * p.D;
-    if (cap && launch_cap(c, 0, n)) return fail(c, TDM_ECUDA, "cap mapping launch failed");
+    if (cap && launch_cap(c, 0, n, false, fields_in)) return fail(c, TDM_ECUDA, "cap mapping launch failed");
     TDM_CU(cudaEventRecord(c->ev_stage[3], c->stream));
     Buffers& b = c->b;
     auto dev_or_stage = [&](auto* user, auto*& stage) -> decltype(user) {
@@ -797,14 +825,16 @@ int tdm_reconstruct(tdm_ctx* c, const float* fields_in, const int32_t* posspec_i
     const size_t FF = (size_t)c->p.F * c->p.F;
     if ((!fields_in || !posspec_in) && n > c->n_fields)
         return fail(c, TDM_EINVAL, "tdm_reconstruct: fewer fields in the context than requested");
-    if (fields_in && fields_in != reinterpret_cast<const float*>(c->b.fields))
+    const float2* direct = is_direct(c, fields_in) ? reinterpret_cast<const float2*>(fields_in) : nullptr;
+    if (fields_in && !direct && fields_in != reinterpret_cast<const float*>(c->b.fields))
         TDM_CU(cudaMemcpyAsync(c->b.fields, fields_in, n * FF * sizeof(float2), cudaMemcpyDefault, c->stream));
     if (posspec_in) {
         if (int rc = set_posspec(c, posspec_in, n, "tdm_reconstruct")) return rc;
         c->n_fields = std::max(c->n_fields, n);
     }
     TDM_CU(cudaEventRecord(c->ev_stage[2], c->stream));
-    int rc = run_volume(c, n, true, indice_out, absorption_out, otf_out, counts_out);
+    int rc = run_volume(c, n, true, indice_out, absorption_out, otf_out, counts_out, true, nullptr, nullptr, nullptr,
+                        nullptr, direct);
     if (rc) return rc;
     c->n_caps = n;
     if (fields_in && !is_device_ptr(fields_in)) return tdm_synchronize(c);

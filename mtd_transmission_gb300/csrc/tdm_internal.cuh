@@ -215,7 +215,17 @@ inline int angles_per_launch(const tdm_ctx* c, int n) {
 // With argmax = true (n at most one chunk), the column pass also leaves the
 // specular search's partial winners of each angle in b.argpart; the return
 // value is then the number of partial records per angle (> 0).
-int launch_extract(tdm_ctx* c, const void* holos_dev, int bits, int n, int a0, bool argmax = false);
+// also (may be null): a second destination of the n spectra.
+int launch_extract(tdm_ctx* c, const void* holos_dev, int bits, int n, int a0, bool argmax = false,
+                   float2* also = nullptr);
+// The caller's device buffers of a field stage, for its n angles: spectra that
+// the specular search reads and copies to the context (its first pass over
+// them), fields that the formation stores beside the context's.  Either may be
+// null: the context's spectra, and no second destination.
+struct FieldIo {
+    const float2* spectra = nullptr;
+    float2* fields = nullptr;
+};
 // Per-angle field formation for spectra [a0, a0 + n).  argparts > 0: the
 // extraction left that many partial winners per angle (one chunk only);
 // form = false (C_ABER pipeline): the fields are formed by the cap row pass.
@@ -223,25 +233,27 @@ int launch_extract(tdm_ctx* c, const void* holos_dev, int bits, int n, int a0, b
 // b.unwrapped), stack angles a0 .. a0 + m - 1; F <= 256.
 int launch_herraez(tdm_ctx* c, int a0, int m);
 int launch_fields(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapped, float* dbg_amp,
-                  int argparts = 0, bool form = true);
+                  int argparts = 0, bool form = true, FieldIo io = {});
 // Per-field spectra and cap contributions for fields [a0, a0 + n); with
 // form = true (one chunk, after launch_fields(..., form = false)) the fields
 // are formed from the chunk's unwrapped phase, amplitude and fits on the fly
 // (and stored in b.fields).
-int launch_cap(tdm_ctx* c, int a0, int n, bool form = false);
+// fields_in (may be null): the caller's fields, read instead of b.fields and
+// copied there.
+int launch_cap(tdm_ctx* c, int a0, int n, bool form = false, const float2* fields_in = nullptr);
 // The same two stages for field sizes that are not powers of two (the
 // mixed-radix engine, fft_generic.cuh; k_generic.cu).
 int launch_fields_generic(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapped, float* dbg_amp,
-                          int argparts, bool form);
-int launch_cap_generic(tdm_ctx* c, int a0, int n, bool form);
+                          int argparts, bool form, FieldIo io);
+int launch_cap_generic(tdm_ctx* c, int a0, int n, bool form, const float2* fields_in);
 // Field sizes the mixed-radix passes are compiled for (2 NXMAX, not powers of two).
 bool generic_field_size(int F);
 // Pieces of the field stage shared by both engines (k_fields.cu): the
 // standalone specular-search partials of m spectra (returns the records per
-// angle), the aberration fits and the field formation of the chunk's m angles.
-int launch_argmax_part(tdm_ctx* c, const float2* spec, int m);
+// angle; copy, if not null, receives the spectra), the aberration fits and the field formation of the chunk's m angles.
+int launch_argmax_part(tdm_ctx* c, const float2* spec, int m, float2* copy);
 void launch_aber_fit(tdm_ctx* c, const float* unw, int m);
-void launch_form(tdm_ctx* c, const float* unw, int g0, int m);
+void launch_form(tdm_ctx* c, const float* unw, int g0, int m, float2* also);
 // Outputs of the volume stage: the device buffers the kernels write and, for
 // each caller buffer in host memory, the host destination its device copy is
 // downloaded to on the copy stream as soon as the pass that completes it has

@@ -109,7 +109,7 @@ int run(const Symbols& s, const void* holos, int bits, int n, float2* out, int F
             static_cast<const char*>(holos) + h0 * in_bytes, bits, s.window + window_offset(H), nullptr, s.twiddle,
             s.scratch, F, x0, nullptr, 0u);
         k_extract_cols<H><<<C::grid_cols(F, m), C::Cols::NT, sm_cols, st>>>(
-            s.scratch, s.twiddle, out + (size_t)h0 * F * F, F, x0, y0, nullptr);
+            s.scratch, s.twiddle, out + (size_t)h0 * F * F, nullptr, F, x0, y0, nullptr);
     }
     return cudaGetLastError() == cudaSuccess ? TDM_OK : TDM_ECUDA;
 }
