@@ -34,12 +34,12 @@
 #include "form.cuh"
 #include "argmax.cuh"
 #include "phase_mean.cuh"
+#include "phasor.cuh"
 
 namespace tdm {
 namespace {
 
 constexpr float kTwoPi = 6.283185307179586f;
-constexpr float kInvTwoPi = 0.15915494309189535f;
 
 template <class K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
@@ -122,38 +122,6 @@ k_field_rows(const float2* __restrict__ spectra, const float4* __restrict__ argp
         for (int k2 = 0; k2 < T; ++k2) dst[j + q * T + E * k2] = x[q * T + k2];
     }
 }
-
-// Amplitude |u| and unit phasor u/|u| (1 where u = 0: atan2(0, 0) = 0) from one
-// reciprocal square root: |u|^2 r, corrected by a Newton step of the square
-// root, and u r.  A field value whose square leaves the normal range is scaled
-// first.
-__device__ __forceinline__ float amplitude(float2 u, float2& z) {
-    auto unit = [&](float2 w) {
-        const float m2 = fmaf(w.x, w.x, w.y * w.y), r = rsqrtf(m2), m = m2 * r;
-        z = make_float2(w.x * r, w.y * r);
-        return fmaf(fmaf(-m, m, m2), 0.5f * r, m);
-    };
-    const float m2 = fmaf(u.x, u.x, u.y * u.y);
-    if (m2 > 1e-30f && m2 < 1e30f) return unit(u);
-    const float m = hypotf(u.x, u.y);
-    if (m > 0.0f && m < __int_as_float(0x7f800000)) {
-        const float k = m < 1.0f ? 0x1p100f : 0x1p-100f;
-        unit(make_float2(u.x * k, u.y * k));
-    } else {
-        z = m == 0.0f ? make_float2(1.0f, 0.0f) : make_float2(u.x / m, u.y / m);
-    }
-    return m;
-}
-
-// What the column pass leaves per field pixel.  FIELD (C_ABER off): the field
-// itself is the result.  The rest leave the amplitude and, for Volkov, the unit
-// phasor; for Herraez or no unwrapping, the wrapped phase.  Volkov's solve
-// gives the unwrapped phase less the wrapped phase's mean, a constant that the
-// aberration fit's constant term takes out of the field, so the phase is formed
-// only where the unwrapped phase itself is wanted (VOLKOV_PHASE), with each CTA's
-// sum of it in psum[a * kPhaseParts + blockIdx.x] (FP32 per thread and warp, FP64
-// across the warps in a fixed order).
-enum FieldMode { FIELD, PHASE, VOLKOV, VOLKOV_PHASE };
 
 // Columns (ColFFT).  Bound by issue: 100 angles of 256^2 35 us with atan2, hypot
 // and two divisions a pixel, 22 us as VOLKOV.
@@ -332,13 +300,6 @@ struct RCfg {
     static constexpr size_t SMEM = (size_t)B * W::STRIDE * sizeof(float2);
 };
 
-// Re(-i g / Z) / 2pi for a unit phasor Z: g conj(Z) / |Z|^2, where |Z|^2 = 1 + d
-// with d a few roundings, so 1 / |Z|^2 is 2 - |Z|^2 to d^2 (the division took a
-// fifth of the row pass: 100 angles of 256^2 32 -> 27 us).
-__device__ __forceinline__ float phasor_gradient(float2 g, float2 z) {
-    return (g.y * z.x - g.x * z.y) * (2.0f - fmaf(z.x, z.x, z.y * z.y)) * kInvTwoPi;
-}
-
 // Pass 1: rows of the mirror.  Mirror rows Y and L-1-Y are the same image
 // row, and only the right half of the phasor's gradient
 // gx = Re(-i dZ/dx / Z) / 2pi is kept: gx[Y][X] = sign(X) gxh[m(Y)][m(X)].
@@ -462,7 +423,7 @@ __device__ __forceinline__ void poisson_row(const float2 (&x)[WarpFFT<F>::E], co
             const float kx = (float)k / (float)L;
             const float den = kx * kx + kyv * kyv;
             // A = -Im qu = -e.y / 2, B = Re qv = d.y / 2
-            p[q * T + k2] = den > 0.0f ? (0.5f * s) * (kyv * d.y - kx * e.y) / den : 0.0f;
+            p[q * T + k2] = den > 0.0f ? quotient((0.5f * s) * (kyv * d.y - kx * e.y), den) : 0.0f;
         });
     });
 }

@@ -30,12 +30,12 @@
 #include "form.cuh"
 #include "argmax.cuh"
 #include "phase_mean.cuh"
+#include "phasor.cuh"
 
 namespace tdm {
 namespace {
 
 constexpr float kTwoPiG = 6.283185307179586f;
-constexpr float kInvTwoPiG = 0.15915494309189535f;
 constexpr int kRows = 8;  // warps (rows) per CTA of a row pass
 constexpr int kCols = 8;  // columns (warps) per CTA of a column pass
 
@@ -133,11 +133,10 @@ gk_field_rows(const float2* __restrict__ spectra, const float4* __restrict__ arg
     for (int k = lane; k < F; k += 32) dst[k] = A[k];
 }
 
-// mode 1: phase/amplitude/phasor (C_ABER) and the CTA's sum of the wrapped
-// phase in psum[a * kPhaseParts + blockIdx.x]; mode 0: the field itself.
-template <int F>
+// What k_field_cols leaves in the same mode.
+template <int F, int MODE>
 __global__ void __launch_bounds__(kCols * 32)
-gk_field_cols(const float2* __restrict__ I1, int mode, const float2* __restrict__ wq, float* __restrict__ phase,
+gk_field_cols(const float2* __restrict__ I1, const float2* __restrict__ wq, float* __restrict__ phase,
               float* __restrict__ amp, float2* __restrict__ zph, float2* __restrict__ fields,
               double* __restrict__ psum) {
     extern __shared__ float2 sm[];
@@ -162,18 +161,20 @@ gk_field_cols(const float2* __restrict__ I1, int mode, const float2* __restrict_
         const float2 u = sm[t * 2 * F + y];
         const int yo = wrap_f(y + F / 2, F), xo = wrap_f(x0 + t + F / 2, F);
         const size_t o = ((size_t)a * F + yo) * F + xo;
-        if (mode) {
-            const float m = hypotf(u.x, u.y);
-            const float ph = atan2f(u.y, u.x);
-            phase[o] = ph;
-            acc += ph;
-            amp[o] = m;
-            zph[o] = m > 0.0f ? make_float2(u.x / m, u.y / m) : make_float2(1.0f, 0.0f);
-        } else {
+        if constexpr (MODE == FIELD) {
             fields[o] = u;
+        } else {
+            float2 z;
+            amp[o] = amplitude(u, z);
+            if constexpr (MODE != PHASE) zph[o] = z;
+            if constexpr (MODE != VOLKOV) {
+                const float ph = atan2f(u.y, u.x);
+                phase[o] = ph;
+                acc += ph;
+            }
         }
     }
-    if (mode) phase_sum_cta<kCols * 32>(acc, psum + (size_t)a * kPhaseParts + blockIdx.x);
+    if constexpr (MODE == VOLKOV_PHASE) phase_sum_cta<kCols * 32>(acc, psum + (size_t)a * kPhaseParts + blockIdx.x);
 }
 
 // ---------------------------------------------------------------- Volkov unwrap
@@ -201,7 +202,7 @@ gk_volkov_rows(const float2* __restrict__ zph, const float2* __restrict__ wq, fl
         lane, [&](int x) { return zr[x]; },
         [&](int x, float2 z) {
             const float2 g = A[x];
-            out[x] = (g.y * z.x - g.x * z.y) / (z.x * z.x + z.y * z.y) * kInvTwoPiG;  // Re(-i g / Z) / 2pi
+            out[x] = phasor_gradient(g, z);
         });
 }
 
@@ -250,7 +251,7 @@ gk_volkov_cols(const float2* __restrict__ zph, const float* __restrict__ gxh, co
             const int c = i % kCols, y = i / kCols;
             if (x0 + c >= F) return;
             const float2 g = arr(c)[y];
-            const float gy = (g.y * v.x - g.x * v.y) / (v.x * v.x + v.y * v.y) * kInvTwoPiG;
+            const float gy = phasor_gradient(g, make_float2(v.x, v.y));
             arr(c)[F + gslot(y, F)] = make_float2(v.z, (y & 1) ? -gy : gy);
         });
     __syncthreads();
@@ -304,7 +305,7 @@ gk_volkov_integ_rows(const float2* __restrict__ cdct, const float2* __restrict__
             const float2 e = c_mul(wk, make_float2(v.x + vm.x, v.y - vm.y));  // 2 qu
             const float2 d = c_mul(wk, make_float2(v.x - vm.x, v.y + vm.y));  // 2i qv
             const float kx = (float)k / (float)L, den = kx * kx + kyv * kyv;
-            const float pk = den > 0.0f ? (0.5f * sc) * (kyv * d.y - kx * e.y) / den : 0.0f;
+            const float pk = den > 0.0f ? quotient((0.5f * sc) * (kyv * d.y - kx * e.y), den) : 0.0f;
             reinterpret_cast<float*>(&P[k])[h] = pk;
         }
         __syncwarp();  // every lane has read A before the next row overwrites it
@@ -337,7 +338,7 @@ gk_volkov_integ_cols(const float* __restrict__ urows, const double* __restrict__
     const int a = blockIdx.y, c0 = blockIdx.x * NC;
     auto pair = [&](int t) { return sm + t * 3 * F + 2 * F; };  // warp t's column pair
     __shared__ float s_mean;
-    if (threadIdx.x == 0) s_mean = phase_mean(psum + (size_t)a * kPhaseParts, nps, F);  // ordered by the barriers below
+    if (threadIdx.x == 0) s_mean = nps ? phase_mean(psum + (size_t)a * kPhaseParts, nps, F) : 0.0f;  // ordered by the barriers below
     staged_copy<NC * F, kCols * 32>(
         threadIdx.x,
         [&](int i) {
@@ -463,7 +464,10 @@ int gfields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapp
     const size_t sm_vrows = warp_arrays(F, kVRows), sm_vcols = warp_arrays(F, kCols);
     static_assert((F + kCols - 1) / kCols <= kPhaseParts, "phase sums per angle");
     const size_t sm_irows = (size_t)kRows * 3 * F * sizeof(float2), sm_icols = (size_t)kCols * 3 * F * sizeof(float2);
-    if (allow_smem(gk_field_rows<F>, sm_rows) || allow_smem(gk_field_cols<F>, sm_cols) ||
+    const bool volkov = p.deroul && p.volkov, mean = volkov && (dbg_phase || dbg_unwrapped);
+    auto field_cols = !p.c_aber ? gk_field_cols<F, FIELD> : mean ? gk_field_cols<F, VOLKOV_PHASE>
+                      : volkov ? gk_field_cols<F, VOLKOV> : gk_field_cols<F, PHASE>;
+    if (allow_smem(gk_field_rows<F>, sm_rows) || allow_smem(field_cols, sm_cols) ||
         allow_smem(gk_volkov_rows<F>, sm_vrows) || allow_smem(gk_volkov_cols<F>, sm_vcols) ||
         allow_smem(gk_volkov_integ_rows<F>, sm_irows) || allow_smem(gk_volkov_integ_cols<F>, sm_icols))
         return TDM_ECUDA;
@@ -481,8 +485,8 @@ int gfields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapp
         }
         {
             Launch l(c, K_FIELD_COLS);
-            gk_field_cols<F><<<dim3(cols, m), kCols * 32, sm_cols, c->stream>>>(
-                b.I1, p.c_aber, b.wq, b.phase, b.amp, b.zph, b.fields + (size_t)g0 * FF, b.phase_sum);
+            field_cols<<<dim3(cols, m), kCols * 32, sm_cols, c->stream>>>(
+                b.I1, b.wq, b.phase, b.amp, b.zph, b.fields + (size_t)g0 * FF, b.phase_sum);
         }
         if (!p.c_aber) continue;
         const float* unw = b.phase;
@@ -508,7 +512,7 @@ int gfields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapp
             {
                 Launch l(c, K_VOLKOV_INTEG_COLS);
                 gk_volkov_integ_cols<F><<<dim3((F + 2 * kCols - 1) / (2 * kCols), m), kCols * 32, sm_icols,
-                                          c->stream>>>(urows, b.phase_sum, (int)cols, b.wq, b.unwrapped);
+                                          c->stream>>>(urows, b.phase_sum, mean ? (int)cols : 0, b.wq, b.unwrapped);
             }
             unw = b.unwrapped;
         }
