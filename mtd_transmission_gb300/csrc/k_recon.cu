@@ -419,10 +419,11 @@ k_gather(const float2* __restrict__ rec, const int16_t* __restrict__ recz, const
 
 // ---------------------------------------------------------------- 3D FFT passes
 // Column passes (y, z): ColFFT, 16 consecutive x a CTA.  Bound by HBM: 512^3
-// with a band of 220, x 137 us and y 144 us (6.7 and 6.4 TB/s), z 337 us
-// (4.5 TB/s, most of it stores); over all planes and staged through shared memory
+// with a band of 220, x 137 us and y 144 us (6.7 and 6.4 TB/s), z 293 us
+// (5.2 TB/s, most of it stores); over all planes and staged through shared memory
 // y and x took 405 and 432 us.  8 columns leave 32-byte pieces in the z pass's
 // stores (713 us), 32 one CTA an SM (y 182, z 352 us).
+
 // Row pass (x): a warp per G rows, registers to registers.
 template <int D>
 struct RowPass {
@@ -498,6 +499,17 @@ k_ypass(float2* __restrict__ vol, const float2* __restrict__ tw, Params p) {
     }
 }
 
+// The z pass's stores: a volume well beyond L2, which its reader cannot find there
+// again, is stored to be evicted first and leaves the cache to the planes that are
+// read (512^3 325 -> 293 us; 1024^3 3.29 ms before, 3.22 to 3.34 after).  It gave
+// nothing to the x and y passes (x 138 -> 134, y 141 -> 143 us), whose 461 MB the
+// next pass reads.
+template <int D>
+__device__ __forceinline__ void put(float* q, float v) {
+    if constexpr (D >= 512) __stcs(q, v);
+    else *q = v;
+}
+
 // Inverse FFT along z of the band (zero elsewhere), scaled and
 // sign-modulated, written as the index (real) and absorption (imaginary)
 // volumes, x fastest, for rows y0 + blockIdx.y.
@@ -526,8 +538,8 @@ k_zpass(const float2* __restrict__ vol, const float2* __restrict__ tw, Params p,
 #pragma unroll
         for (int k2 = 0; k2 < T; ++k2) {
             const size_t z = j + q * T + E * k2;
-            if (re) re[z * D * D + o] = x[q * T + k2].x * sg;
-            if (im) im[z * D * D + o] = x[q * T + k2].y * sg;
+            if (re) put<D>(&re[z * D * D + o], x[q * T + k2].x * sg);
+            if (im) put<D>(&im[z * D * D + o], x[q * T + k2].y * sg);
         }
     }
 }
