@@ -115,18 +115,18 @@ __device__ __forceinline__ float2 twc(float2 v) {
     }
 }
 
-template <int R, int DIR>
-__device__ __forceinline__ void dft(float2* x);
+template <int R, int DIR, class V>
+__device__ __forceinline__ void dft(V* x);
 
 // R = N1 N2: N2 DFTs of N1 points on the stride-N2 subsequences, twiddles
 // W_R^(n2 k1), N1 DFTs of N2 points; X[k1 + N1 k2].
-template <int N1, int N2, int DIR>
-__device__ __forceinline__ void dft_split(float2* x) {
+template <int N1, int N2, int DIR, class V>
+__device__ __forceinline__ void dft_split(V* x) {
     constexpr int R = N1 * N2;
-    float2 y[R];
+    V y[R];
     static_for<0, N2>([&](auto n2c) {
         constexpr int n2 = decltype(n2c)::value;
-        float2 t[N1];
+        V t[N1];
 #pragma unroll
         for (int n1 = 0; n1 < N1; ++n1) t[n1] = x[N2 * n1 + n2];
         dft<N1, DIR>(t);
@@ -137,7 +137,7 @@ __device__ __forceinline__ void dft_split(float2* x) {
     });
 #pragma unroll
     for (int k1 = 0; k1 < N1; ++k1) {
-        float2 t[N2];
+        V t[N2];
 #pragma unroll
         for (int n2 = 0; n2 < N2; ++n2) t[n2] = y[n2 * N1 + k1];
         dft<N2, DIR>(t);
@@ -146,8 +146,8 @@ __device__ __forceinline__ void dft_split(float2* x) {
     }
 }
 
-template <int R, int DIR>
-__device__ __forceinline__ void dft(float2* x) {
+template <int R, int DIR, class V>
+__device__ __forceinline__ void dft(V* x) {
     if constexpr (R == 2) dft2<DIR>(x[0], x[1]);
     else if constexpr (R == 4) dft4<DIR>(x[0], x[1], x[2], x[3]);
     else if constexpr (R == 8) dft8<DIR>(x);
@@ -177,8 +177,8 @@ struct WarpFFT {
 // W^(j (8a + b)) = W^(8ja) W^(jb) is formed in registers: 7 + E/8 - 1 loads
 // instead of E - 1 (the loads' L1 latency, not their arithmetic, bounded the
 // FFT passes), at about one extra rounding per factor.
-template <int N, int DIR>
-__device__ __forceinline__ void twiddle_lane(float2 (&x)[WarpFFT<N>::E], const float2* __restrict__ twr, int j) {
+template <int N, int DIR, class V>
+__device__ __forceinline__ void twiddle_lane(V (&x)[WarpFFT<N>::E], const float2* __restrict__ twr, int j) {
     using W = WarpFFT<N>;
     constexpr int E = W::E, T = W::T;
     constexpr int R = E >= 16 ? 8 : E;  // k1 = R a + b
@@ -203,8 +203,8 @@ __device__ __forceinline__ void twiddle_lane(float2 (&x)[WarpFFT<N>::E], const f
 // return x[q T + k2] holds element (j + q T) + E k2.  s is the transform's
 // padded shared-memory array (WarpFFT<N>::LEN slots), used for the exchange.
 // Every lane of the warp must call it together.
-template <int N, int DIR>
-__device__ __forceinline__ void fft_warp_regs(float2 (&x)[WarpFFT<N>::E], float2* s, int j,
+template <int N, int DIR, class V>
+__device__ __forceinline__ void fft_warp_regs(V (&x)[WarpFFT<N>::E], float2* s, int j,
                                               const float2* __restrict__ tw) {
     using W = WarpFFT<N>;
     constexpr int E = W::E, T = W::T;
@@ -251,8 +251,8 @@ struct ColFFT {
 // fft_warp_regs and fft_warp_regs_rev for such a pass (s: the column's array).
 // FIRST: nothing in s is still to be read by other threads on entry.
 // Every thread of the CTA calls them together.
-template <int N, int DIR, bool FIRST = true>
-__device__ __forceinline__ void fft_cta_regs(float2 (&x)[WarpFFT<N>::E], float2* s, int j,
+template <int N, int DIR, bool FIRST = true, class V>
+__device__ __forceinline__ void fft_cta_regs(V (&x)[WarpFFT<N>::E], float2* s, int j,
                                              const float2* __restrict__ tw) {
     using W = WarpFFT<N>;
     constexpr int E = W::E, T = W::T;

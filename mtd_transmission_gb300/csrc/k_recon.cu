@@ -60,7 +60,7 @@ k_cap_rows(const float2* __restrict__ fields, const float* __restrict__ tuk, int
     const int a = blockIdx.y, y = blockIdx.x * C::B + tr;
     const float wy = tuk[y];
     const float2* src = fields + ((size_t)a * F + y) * F;
-    float2 x[E];
+    Fusable x[E];
 #pragma unroll
     for (int n1 = 0; n1 < E; ++n1) {
         const int xx = j + n1 * T;
@@ -105,13 +105,13 @@ k_cap_rows_form(const float* __restrict__ unwrapped, const float* __restrict__ a
     const float wy = tuk[y];
     const size_t row = ((size_t)a * F + y) * F;
     const FormRow fr = form_row(bf, y, F);
-    float2 x[E];
+    Fusable x[E];
 #pragma unroll
     for (int n1 = 0; n1 < E; ++n1) {
         const int xx = j + n1 * T;
         const float2 f = form_value(fr, xx, F, unwrapped[row + xx], amp[row + xx], born);
         fields[row + xx] = f;
-        x[n1] = c_scale(f, ((xx >= flat.x && xx <= flat.y) ? 1.0f : __ldg(&tuk[xx])) * wy);
+        x[n1] = c_scale(Fusable(f), ((xx >= flat.x && xx <= flat.y) ? 1.0f : __ldg(&tuk[xx])) * wy);
     }
     fft_warp_regs<F, -1>(x, sm + tr * W::STRIDE, j, tw);
     float2* dst = r1 + row;
@@ -145,7 +145,7 @@ k_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, cons
     const CapFz fz = cap_fzm0(p, ps, s_tab, s_pair);
     const float ir = (float)p.inv_rayon;
     const size_t o = (size_t)a * F * F + kx;
-    float2 x[E];
+    Fusable x[E];
 #pragma unroll
     for (int n1 = 0; n1 < E; ++n1) x[n1] = r1[o + (size_t)(j + n1 * T) * F];
     fft_cta_regs<F, -1>(x, sm + t * W::STRIDE, j, tw);
