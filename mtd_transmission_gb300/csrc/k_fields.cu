@@ -86,8 +86,8 @@ struct FieldCfg {
 template <int F>
 __global__ void __launch_bounds__(FieldCfg<F>::NT)
 k_field_rows(const float2* __restrict__ spectra, const float4* __restrict__ argpart, int nparts,
-             int2* __restrict__ posspec, float2* __restrict__ specval, int normalize, const float2* __restrict__ tw,
-             float2* __restrict__ I1) {
+             int2* __restrict__ posspec, int2* __restrict__ also, float2* __restrict__ specval, int normalize,
+             const float2* __restrict__ tw, float2* __restrict__ I1) {
     using C = FieldCfg<F>;
     using W = typename C::W;
     constexpr int T = W::T, E = W::E;
@@ -99,6 +99,7 @@ k_field_rows(const float2* __restrict__ spectra, const float4* __restrict__ argp
     const int2 p = make_int2(bi % F, bi / F);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         posspec[a] = p;
+        if (also) also[a] = p;
         specval[a] = spec[bi];
     }
     float2 nrm = make_float2(1.0f, 0.0f);
@@ -647,7 +648,8 @@ int fields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrappe
         {
             Launch l(c, K_FIELD_ROWS);
             k_field_rows<F><<<dim3(F / FC::B, m), FC::NT, FC::SMEM, c->stream>>>(
-                spec, b.argpart, nparts, b.posspec + g0, b.specval + g0, p.c_aber ? 0 : 1, b.tw, b.I1);
+                spec, b.argpart, nparts, b.posspec + g0, io.posspec ? io.posspec + (g0 - a0) : nullptr,
+                b.specval + g0, p.c_aber ? 0 : 1, b.tw, b.I1);
         }
         {
             Launch l(c, K_FIELD_COLS);

@@ -102,8 +102,8 @@ __device__ __forceinline__ void gmirror_derivative(float2* a, float2* b, const f
 template <int F>
 __global__ void __launch_bounds__(kRows * 32)
 gk_field_rows(const float2* __restrict__ spectra, const float4* __restrict__ argpart, int nparts,
-              int2* __restrict__ posspec, float2* __restrict__ specval, int normalize, const float2* __restrict__ wq,
-              float2* __restrict__ I1) {
+              int2* __restrict__ posspec, int2* __restrict__ also, float2* __restrict__ specval, int normalize,
+              const float2* __restrict__ wq, float2* __restrict__ I1) {
     extern __shared__ float2 sm[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int a = blockIdx.y, r = blockIdx.x * kRows + w;
@@ -112,6 +112,7 @@ gk_field_rows(const float2* __restrict__ spectra, const float4* __restrict__ arg
     const int2 p = make_int2(bi % F, bi / F);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         posspec[a] = p;
+        if (also) also[a] = p;
         specval[a] = spec[bi];
     }
     if (r >= F) return;  // warp-uniform, after the CTA-wide search
@@ -481,7 +482,8 @@ int gfields_impl(tdm_ctx* c, int a0, int n, float* dbg_phase, float* dbg_unwrapp
         {
             Launch l(c, K_FIELD_ROWS);
             gk_field_rows<F><<<dim3(rows, m), kRows * 32, sm_rows, c->stream>>>(
-                spec, b.argpart, nparts, b.posspec + g0, b.specval + g0, p.c_aber ? 0 : 1, b.wq, b.I1);
+                spec, b.argpart, nparts, b.posspec + g0, io.posspec ? io.posspec + (g0 - a0) : nullptr,
+                b.specval + g0, p.c_aber ? 0 : 1, b.wq, b.I1);
         }
         {
             Launch l(c, K_FIELD_COLS);

@@ -876,8 +876,8 @@ static void use_scratch(tdm_ctx* c, const ChunkScratch& k) {
 // each lane a stream with its own chunk slots of the scratch buffers, forked
 // from the context stream and joined back at the end.  The launchers read
 // c->stream and the scratch pointers, which are switched per chunk here and
-// restored on every return.
-static int stage_angles(tdm_ctx* c, const void* holos, int bits, int n) {
+// restored on every return.  The specular positions also go to pos.
+static int stage_angles(tdm_ctx* c, const void* holos, int bits, int n, int2* pos) {
     const Params& p = c->p;
     const size_t per = (size_t)p.H * p.H * (bits == 16 ? 2 : 1);
     const bool dev = is_device_ptr(holos);
@@ -931,7 +931,9 @@ static int stage_angles(tdm_ctx* c, const void* holos, int bits, int n) {
         if (parts <= 0) return fail(c, parts ? parts : TDM_ECUDA, "extraction launch failed");
         if (!dev) TDM_CU(cudaEventRecord(c->ev_free[buf], c->stream));
         const bool form_in_cap = p.c_aber != 0;
-        if (int rc = launch_fields(c, h0, m, nullptr, nullptr, nullptr, parts, !form_in_cap))
+        FieldIo io;
+        io.posspec = pos + h0;
+        if (int rc = launch_fields(c, h0, m, nullptr, nullptr, nullptr, parts, !form_in_cap, io))
             return fail(c, rc, "fields launch failed");
         if (int rc = launch_cap(c, h0, m, form_in_cap)) return fail(c, rc, "cap mapping launch failed");
     }
@@ -950,7 +952,7 @@ static int pipeline(tdm_ctx* c, const void* holos, int bits, int n, float* indic
     // The per-angle stages run on c->stream, the volume stage on vol_stream, so
     // that this call's volume stage overlaps the next call's per-angle stages.
     // This call's cap records go to rec_buf[par], after the gather of two calls
-    // ago has read it; the specular positions its gather reads are copied aside.
+    // ago has read it, and the specular positions that its gather reads to posspec_vol[par].
     const int par = c->rec_parity;
     c->b.rec = c->b.rec_buf[par];
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -958,7 +960,7 @@ static int pipeline(tdm_ctx* c, const void* holos, int bits, int n, float* indic
     const bool capturing = cap != cudaStreamCaptureStatusNone;
     if (!capturing) TDM_CU(cudaStreamWaitEvent(c->stream, c->ev_rec_free[par], 0));  // a graph is ordered by its launches
     TDM_CU(cudaEventRecord(c->ev_stage[0], c->stream));
-    if (int rc = stage_angles(c, holos, bits, n)) return rc;
+    if (int rc = stage_angles(c, holos, bits, n, c->b.posspec_vol[par])) return rc;
     TDM_CU(cudaEventRecord(c->ev_stage[1], c->stream));  // extract, fields and map are interleaved
     TDM_CU(cudaEventRecord(c->ev_stage[2], c->stream));
     c->n_spectra = n;
@@ -968,8 +970,6 @@ static int pipeline(tdm_ctx* c, const void* holos, int bits, int n, float* indic
         Launch l(c, K_POSSPEC);
         k_unpack_posspec<<<(n + 255) / 256, 256, 0, c->stream>>>(c->b.posspec, n, posspec_out);
     }
-    TDM_CU(cudaMemcpyAsync(c->b.posspec_vol[par], c->b.posspec, n * sizeof(int2), cudaMemcpyDeviceToDevice,
-                           c->stream));
     TDM_CU(cudaEventRecord(c->ev_angles, c->stream));
     TDM_CU(cudaStreamWaitEvent(c->vol_stream, c->ev_angles, 0));
     int rc = run_volume(c, n, false, indice_out, absorption_out, otf_out, counts_out, wait, c->vol_stream,

@@ -218,13 +218,15 @@ inline int angles_per_launch(const tdm_ctx* c, int n) {
 // also (may be null): a second destination of the n spectra.
 int launch_extract(tdm_ctx* c, const void* holos_dev, int bits, int n, int a0, bool argmax = false,
                    float2* also = nullptr);
-// The caller's device buffers of a field stage, for its n angles: spectra that
-// the specular search reads and copies to the context (its first pass over
-// them), fields that the formation stores beside the context's.  Either may be
-// null: the context's spectra, and no second destination.
+// Device buffers of a field stage beside the context's, for its n angles:
+// the caller's spectra, which the specular search reads and copies to the context
+// (its first pass over them), and second destinations of the fields (the
+// caller's) and of the specular positions (those that a pipeline call's volume
+// stage reads).  Each may be null: the context's spectra, no second destination.
 struct FieldIo {
     const float2* spectra = nullptr;
     float2* fields = nullptr;
+    int2* posspec = nullptr;
 };
 // Per-angle field formation for spectra [a0, a0 + n).  argparts > 0: the
 // extraction left that many partial winners per angle (one chunk only);
