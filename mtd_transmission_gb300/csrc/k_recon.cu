@@ -512,17 +512,17 @@ __device__ __forceinline__ void put(float* q, float v) {
 
 // Inverse FFT along z of the band (zero elsewhere), scaled and
 // sign-modulated, written as the index (real) and absorption (imaginary)
-// volumes, x fastest, for rows y0 + blockIdx.y.
+// volumes (either may be null), x fastest.
 template <int D>
 __global__ void __launch_bounds__(ColPass<D>::NT, ColPass<D>::CTAS)
-k_zpass(const float2* __restrict__ vol, const float2* __restrict__ tw, Params p, float scale, int y0,
-        float* __restrict__ re, float* __restrict__ im) {
+k_zpass(const float2* __restrict__ vol, const float2* __restrict__ tw, Params p, float scale, float* __restrict__ re,
+        float* __restrict__ im) {
     using C = ColPass<D>;
     using W = typename C::W;
     constexpr int T = W::T, E = W::E;
     extern __shared__ float2 sm[];
     const int t = C::column(), j = C::adjacent_j();
-    const int X = blockIdx.x * C::B + t, Y = y0 + blockIdx.y;
+    const int X = blockIdx.x * C::B + t, Y = blockIdx.y;
     const float2* col = vol + (size_t)Y * D + X;
     float2 x[E];
 #pragma unroll
@@ -863,8 +863,8 @@ int volume_impl(tdm_ctx* c, int n, const VolumeOut& out, cudaStream_t st, CapRec
     // each part's writer waits for that part's download (ev_dl) just before it runs.
     auto staged_free = [&](int part) { return cudaStreamWaitEvent(st, c->ev_dl[part], 0); };
     auto downloaded = [&](int part) { return cudaEventRecord(c->ev_dl[part], c->dl_stream); };
-    if (out.host_cnt && staged_free(kOutSlabs)) return TDM_ECUDA;
-    if (out.host_otf && staged_free(kOutSlabs + 1)) return TDM_ECUDA;
+    if (out.host_cnt && staged_free(kOutVolumes)) return TDM_ECUDA;
+    if (out.host_otf && staged_free(kOutVolumes + 1)) return TDM_ECUDA;
     // cells outside the cap band and outside the columns that caps reach carry no hits and no OTF support
     const size_t plane = (size_t)D * D, NT = (size_t)D * D * D;
     const bool all = p.xa == 0 && p.xb == D && p.ya == 0 && p.yb == D;
@@ -882,36 +882,36 @@ int volume_impl(tdm_ctx* c, int n, const VolumeOut& out, cudaStream_t st, CapRec
     cudaEventRecord(c->ev_stage[5], st);
     if (ev_gathered && cudaEventRecord(ev_gathered, st)) return TDM_ECUDA;
     if (out.host_cnt) {
-        if (download_after(c, st, c->ev_out[kOutSlabs], out.host_cnt, cnt, NT * sizeof(uint32_t)) ||
-            downloaded(kOutSlabs))
+        if (download_after(c, st, c->ev_out[kOutVolumes], out.host_cnt, cnt, NT * sizeof(uint32_t)) ||
+            downloaded(kOutVolumes))
             return TDM_ECUDA;
     }
     if (out.host_otf) {
-        if (download_after(c, st, c->ev_out[kOutSlabs + 1], out.host_otf, otf, NT) || downloaded(kOutSlabs + 1))
+        if (download_after(c, st, c->ev_out[kOutVolumes + 1], out.host_otf, otf, NT) || downloaded(kOutVolumes + 1))
             return TDM_ECUDA;
     }
     if (int rc = launch_xy<D>(c, st)) return rc;
-    // z pass by slabs of rows y; a slab's rows are final in every plane once it has run
-    const bool host_vol = out.host_re || out.host_im;
-    const int nslab = host_vol ? kOutSlabs : 1;
-    for (int sl = 0; sl < nslab; ++sl) {
-        const int y0 = sl * D / nslab, y1 = (sl + 1) * D / nslab;
-        if (host_vol && staged_free(sl)) return TDM_ECUDA;
+    // Two volumes for the host take a z pass each: the second runs while the first
+    // is downloaded, and the next call's first while this call's second is.  Whole
+    // volumes, because the link carries uploads and downloads at once at its full
+    // rate only in contiguous copies (600 x 1024^2 to 512^3 from and to the host,
+    // uploads overlapping: 131.6 volumes/s; one z pass for both by slabs of rows, whose
+    // download is strided, 116).
+    const bool host_vol = out.host_re || out.host_im, split = out.host_re && out.host_im;
+    if (host_vol && !split && (staged_free(0) || staged_free(1))) return TDM_ECUDA;
+    for (int part = 0; part < (split ? 2 : 1); ++part) {
+        if (split && staged_free(part)) return TDM_ECUDA;
         {
             Launch l(c, K_ZPASS, st);
-            k_zpass<D><<<dim3(D / P::B, y1 - y0), P::NT, P::SMEM, st>>>(b.vol, b.tw, p, p.out_scale, y0, re, im);
+            k_zpass<D><<<dim3(D / P::B, D), P::NT, P::SMEM, st>>>(b.vol, b.tw, p, p.out_scale,
+                                                                 split && part ? nullptr : re,
+                                                                 split && !part ? nullptr : im);
         }
         if (host_vol) {
-            const size_t off = (size_t)y0 * D, pitch = plane * sizeof(float), width = (size_t)(y1 - y0) * D * sizeof(float);
-            if (cudaEventRecord(c->ev_out[sl], st) || cudaStreamWaitEvent(c->dl_stream, c->ev_out[sl], 0))
+            const int q = part || !out.host_re;  // the volume that goes to the host
+            if (download_after(c, st, c->ev_out[q], q ? out.host_im : out.host_re, q ? im : re, NT * sizeof(float)) ||
+                downloaded(q))
                 return TDM_ECUDA;
-            if (out.host_re && cudaMemcpy2DAsync(out.host_re + off, pitch, re + off, pitch, width, D,
-                                                 cudaMemcpyDeviceToHost, c->dl_stream))
-                return TDM_ECUDA;
-            if (out.host_im && cudaMemcpy2DAsync(out.host_im + off, pitch, im + off, pitch, width, D,
-                                                 cudaMemcpyDeviceToHost, c->dl_stream))
-                return TDM_ECUDA;
-            if (downloaded(sl)) return TDM_ECUDA;
         }
     }
     cudaEventRecord(c->ev_stage[6], st);
@@ -960,7 +960,7 @@ int adjoint_impl(tdm_ctx* c, CapRecs recs, int n, float* xn, float* xk, bool nor
     const float scale = normalize ? p.out_scale : (float)(1.0 / ((double)p.out_scale * (double)D * D * D));
     {
         Launch l(c, K_ZPASS);
-        k_zpass<D><<<dim3(D / P::B, D), P::NT, P::SMEM, c->stream>>>(b.vol, b.tw, p, scale, 0, xn, xk);
+        k_zpass<D><<<dim3(D / P::B, D), P::NT, P::SMEM, c->stream>>>(b.vol, b.tw, p, scale, xn, xk);
     }
     return cudaGetLastError() == cudaSuccess ? TDM_OK : TDM_ECUDA;
 }

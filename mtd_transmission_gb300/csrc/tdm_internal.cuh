@@ -13,8 +13,8 @@
 namespace tdm {
 
 constexpr int kNC = 15;  // degree-4 2D polynomial: 15 monomials
-constexpr int kOutSlabs = 4;  // z-pass slabs (rows y) whose outputs are downloaded while the next slab runs
-constexpr int kOutEvents = kOutSlabs + 2;
+constexpr int kOutVolumes = 2;  // index and absorption, downloaded one after the other
+constexpr int kOutEvents = kOutVolumes + 2;
 constexpr int kMaxLanes = 8;    // chunks of the per-angle stages in flight at once
 constexpr int kStageSlots = 16; // hologram upload slots of one chunk each
 constexpr size_t kL2Bytes = size_t(126) << 20;
@@ -136,7 +136,7 @@ struct tdm_ctx {
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;  // hologram uploads
     cudaStream_t dl_stream = nullptr;    // output downloads (a second copy engine)
-    // downloads of the staged outputs done, per part (z-pass slabs, then counts, then OTF): a volume
+    // downloads of the staged outputs done, per part (index, absorption, counts, OTF): a volume
     // stage waits for the previous volume's download of a part just before it rewrites that part
     cudaEvent_t ev_dl[tdm::kOutEvents] = {};
     // tdm_pipeline runs each volume's stage (gather, z/y/x passes) on vol_stream, so that it
@@ -259,7 +259,7 @@ void launch_form(tdm_ctx* c, const float* unw, int g0, int m, float2* also);
 // Outputs of the volume stage: the device buffers the kernels write and, for
 // each caller buffer in host memory, the host destination its device copy is
 // downloaded to on the copy stream as soon as the pass that completes it has
-// run (the index and absorption volumes slab by slab during the z pass).
+// run (the index volume while the absorption volume is computed).
 struct VolumeOut {
     float* re = nullptr;
     float* im = nullptr;
@@ -288,7 +288,7 @@ int launch_tv_step(tdm_ctx* c, const float* xn, const float* xk, const float* gn
                    float* xk_out);
 // gather of the cap records rec (angles [0, n), specular positions posspec),
 // normalisation and 3D inverse FFT into the outputs, on stream st.  Downloads
-// run on c->dl_stream; each staged part (z-pass slab, counts, OTF) is
+// run on c->dl_stream; each staged part (index, absorption, counts, OTF) is
 // rewritten only after the previous volume's download of that part is done
 // (c->ev_dl).  ev_gathered (may be null) is recorded on st once the gather
 // has read rec.
