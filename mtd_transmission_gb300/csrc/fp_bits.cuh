@@ -1,10 +1,9 @@
 // IEEE 754 binary32 <-> binary64 conversions done with integer operations.
 //
 // The GB300 FP64 pipe runs at a small fraction of the FP32 rate and the
-// hardware conversions between float and double issue on it.  The cap
-// accumulation adds in FP64 but its inputs and outputs are FP32, so it
-// widens every hit and narrows every cell; doing both on the integer pipe
-// leaves the FP64 pipe to the additions.  Both functions give the exact IEEE
+// hardware conversions between float and double issue on it.  The misfit of the
+// forward operator squares and adds FP32 residuals in FP64; widening them on the
+// integer pipe leaves the FP64 pipe to that.  Both functions give the exact IEEE
 // results: widening is exact, narrowing rounds to nearest, ties to even, with
 // subnormal results, overflow to infinity and NaN handled as the standard
 // says.  The header also compiles as plain C++ for the host-side check.
