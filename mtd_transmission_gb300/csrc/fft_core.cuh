@@ -1,16 +1,5 @@
-// Shared-memory Stockham FFT building blocks for sm_103a.
-//
-// A CTA holds B transforms of N points each in shared memory (complex64,
-// padded layout).  Each transform is worked by T = N/8 threads that each keep
-// 8 points in registers per stage: radix-8 stages, then one radix-4 or
-// radix-2 stage for sizes that are not a power of 8.  Stage s with span Ns
-// reads point b + k*N/R, twiddles it by W_{Ns*R}^{(b mod Ns) k}, runs an R-point
-// DFT and writes point (b/Ns)*Ns*R + (b mod Ns) + m*Ns (autosort: natural
-// order in, natural order out, no bit reversal).
-//
-// Layout: logical point i of a transform lives at pad_idx(i) = i + i/16, one
-// spare complex every 16, which spreads the stride-R stores of the early
-// stages over all banks; transforms are tstride(N) (odd) complexes apart.
+// Complex arithmetic and register butterflies of the FFT passes for sm_103a, and
+// the sizes of their twiddle table.
 //
 // Sign conventions follow FFTW: DIR = -1 is exp(-2 pi i jk/N) (forward),
 // DIR = +1 is exp(+2 pi i jk/N) (backward); neither is normalised.
@@ -31,11 +20,6 @@ __host__ __device__ constexpr int warp_fft_e(int n) { return n >= 2048 ? 64 : n 
 __host__ __device__ constexpr int twr_offset(int n) { return kTwN + n - 64; }
 constexpr int kTwTotal = kTwN + 4096 - 64;
 
-__host__ __device__ constexpr int pad_idx(int i) { return i + (i >> 4); }
-__host__ __device__ constexpr int padded_len(int n) { return n + (n >> 4); }
-// Distance between consecutive transforms of a CTA in shared memory: odd, so
-// that B transforms read at the same logical index fall in distinct banks.
-__host__ __device__ constexpr int tstride(int n) { return padded_len(n) + 1; }
 __host__ __device__ constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c(n >> 1); }
 
 // A complex value is a register pair, and the packed FP32 instructions of this
@@ -120,64 +104,6 @@ __device__ __forceinline__ void dft8(V* x) {
     x[6] = make_float2(e2.x + DIR * o2.y, e2.y - DIR * o2.x);
     x[3] = __ffma2_rn(rp, u3, e3);
     x[7] = __ffma2_rn(rm, u3, e3);
-}
-
-// One Stockham stage on a transform held in shared memory (in place).
-// Every thread of the CTA must call it (it contains __syncthreads()); threads
-// with active == false only take part in the barriers.
-template <int N, int R, int NS, int DIR>
-__device__ __forceinline__ void fft_stage(float2* s, int j, const float2* __restrict__ tw, bool active) {
-    constexpr int T = N / 8;
-    constexpr int NB = 8 / R;
-    float2 x[8];
-    if (active) {
-#pragma unroll
-        for (int t = 0; t < NB; ++t) {
-            const int b = j + t * T;
-#pragma unroll
-            for (int k = 0; k < R; ++k) x[t * R + k] = s[pad_idx(b + k * (N / R))];
-        }
-    }
-    __syncthreads();
-    if (active) {
-#pragma unroll
-        for (int t = 0; t < NB; ++t) {
-            const int b = j + t * T;
-            const int p = b % NS;
-            if constexpr (NS > 1) {
-#pragma unroll
-                for (int k = 1; k < R; ++k) {
-                    float2 w = __ldg(&tw[p * k * (kTwN / (NS * R))]);
-                    if constexpr (DIR > 0) w.y = -w.y;
-                    x[t * R + k] = c_mul(x[t * R + k], w);
-                }
-            }
-            if constexpr (R == 8) dft8<DIR>(&x[t * R]);
-            else if constexpr (R == 4) dft4<DIR>(x[t * R], x[t * R + 1], x[t * R + 2], x[t * R + 3]);
-            else dft2<DIR>(x[t * R], x[t * R + 1]);
-            const int base = (b / NS) * NS * R + p;
-#pragma unroll
-            for (int m = 0; m < R; ++m) s[pad_idx(base + m * NS)] = x[t * R + m];
-        }
-    }
-    __syncthreads();
-}
-
-// Full N-point transform of the padded shared-memory array s, worked by
-// thread j in [0, N/8) of the transform.  Input and output in natural order.
-template <int N, int DIR>
-__device__ __forceinline__ void fft_smem(float2* s, int j, const float2* __restrict__ tw, bool active = true) {
-    static_assert(N >= 64 && N <= kTwN && (N & (N - 1)) == 0, "power-of-two size in [64, 4096]");
-    constexpr int L2 = ilog2c(N);
-    constexpr int n8 = L2 / 3;
-    constexpr int rem = L2 % 3;
-    fft_stage<N, 8, 1, DIR>(s, j, tw, active);
-    fft_stage<N, 8, 8, DIR>(s, j, tw, active);
-    if constexpr (n8 >= 3) fft_stage<N, 8, 64, DIR>(s, j, tw, active);
-    if constexpr (n8 >= 4) fft_stage<N, 8, 512, DIR>(s, j, tw, active);
-    constexpr int NSf = 1 << (3 * n8);
-    if constexpr (rem == 1) fft_stage<N, 2, NSf, DIR>(s, j, tw, active);
-    if constexpr (rem == 2) fft_stage<N, 4, NSf, DIR>(s, j, tw, active);
 }
 
 }  // namespace tdm

@@ -321,72 +321,12 @@ __device__ __forceinline__ void fft_warp_regs_rev(float2 (&x)[WarpFFT<N>::E], fl
     dft<E, DIR>(x);
 }
 
-// Forward transform with sign DIR, x[k] *= mul(k, x[k]) for every bin k, and
-// the unnormalised transform with sign -DIR; x in the input order of
-// fft_warp_regs on entry and on return.
-template <int N, int DIR, class Mul>
-__device__ __forceinline__ void fft_warp_filter(float2 (&x)[WarpFFT<N>::E], float2* s, int j,
-                                                const float2* __restrict__ tw, Mul&& mul) {
-    using W = WarpFFT<N>;
-    constexpr int E = W::E, T = W::T;
-    fft_warp_regs<N, DIR>(x, s, j, tw);
-#pragma unroll
-    for (int q = 0; q < E / T; ++q) {
-#pragma unroll
-        for (int k2 = 0; k2 < T; ++k2) x[q * T + k2] = mul(j + q * T + E * k2, x[q * T + k2]);
-    }
-    fft_warp_regs_rev<N, -DIR>(x, s, j, tw);
-}
-
 // Position in the padded array of element (j + q T) + E k2, the element held
 // in register q T + k2 after fft_warp_regs.
 template <int N>
 __device__ __forceinline__ int warp_out_pos(int j, int q, int k2) {
     using W = WarpFFT<N>;
     return j + q * W::T + W::E * k2 + q + (W::E / W::T) * k2;
-}
-
-// Shared-memory form: transforms the padded array s in place (natural order
-// in and out).  The caller orders other threads' accesses to s around it.
-template <int N, int DIR>
-__device__ __forceinline__ void fft_warp(float2* s, int j, const float2* __restrict__ tw) {
-    using W = WarpFFT<N>;
-    constexpr int E = W::E, T = W::T;
-    float2 x[E];
-#pragma unroll
-    for (int n1 = 0; n1 < E; ++n1) x[n1] = s[j + n1 * (T + 1)];  // pad(j + T n1)
-    fft_warp_regs<N, DIR>(x, s, j, tw);
-    __syncwarp();
-#pragma unroll
-    for (int q = 0; q < E / T; ++q) {
-#pragma unroll
-        for (int k2 = 0; k2 < T; ++k2) s[warp_out_pos<N>(j, q, k2)] = x[q * T + k2];
-    }
-}
-
-// Out-of-line copy of fft_warp: one body per (N, DIR) however many call
-// sites a kernel has, which bounds the code size and the register count of
-// kernels that chain several transforms.
-template <int N, int DIR>
-__device__ __noinline__ void fft_warp_call(float2* s, int j, const float2* __restrict__ tw) {
-    fft_warp<N, DIR>(s, j, tw);
-}
-
-// Shared-memory filter on the out-of-line transforms: s (natural order) is
-// replaced by FFT_{-DIR}(mul(k, FFT_DIR(s)[k])), unnormalised.
-template <int N, int DIR, class Mul>
-__device__ __forceinline__ void fft_warp_filter_call(float2* s, int j, const float2* __restrict__ tw, Mul&& mul) {
-    using W = WarpFFT<N>;
-    constexpr int E = W::E, T = W::T;
-    fft_warp_call<N, DIR>(s, j, tw);
-    __syncwarp();
-#pragma unroll 8
-    for (int n1 = 0; n1 < E; ++n1) {
-        float2* p = &s[j + n1 * (T + 1)];  // pad(j + T n1)
-        *p = mul(j + n1 * T, *p);
-    }
-    __syncwarp();
-    fft_warp_call<N, -DIR>(s, j, tw);
 }
 
 }  // namespace tdm
