@@ -30,6 +30,7 @@
 #include "form.cuh"
 #include "fp_bits.cuh"
 #include "cap_geometry.cuh"
+#include "gather_smem.cuh"
 
 namespace tdm {
 namespace {
@@ -207,14 +208,6 @@ k_cap_cols(const float2* __restrict__ r1, const int2* __restrict__ posspec, cons
 // one after the other in ascending angle order, so the sums are deterministic;
 // the hit counts are exact.
 
-// A listed angle: its specular x and its index.  Both fit 16 bits: an angle is
-// listed only when its window meets the CTA's columns, which bounds x by the
-// volume's side, and a stack has at most 65535 angles.
-struct Listed {
-    int16_t x;
-    uint16_t angle;
-};
-
 // Lists, in ascending order, the angles whose window covers row Y (by = Y -
 // D/2) and one of the columns bx0 .. bx0 + nx - 1 of the CTA.  Returns the
 // count; all NW warps of the CTA call it together, and it ends with a barrier.
@@ -327,25 +320,6 @@ __device__ __forceinline__ float over(float x, float n, float r) {
 // sums of FP32 group sums, and each lane loading its angle's records, 538); 400
 // of 128^2 to 256^3 76 us (100).
 template <int W>
-struct GatherSmem {
-    // per warp: sums, counts (uint16) and cells with a hit (uint16), at a pitch of
-    // 16 bytes mod 128: with the normalised cell of an odd plane in the upper half of its sums' slot, the
-    // CTA-wide store's reads fall in distinct banks.  Per CTA: two tiles of 32
-    // angles' cells (odd row pitches, so that a column is read without
-    // conflicts) and the list of angles.
-    static constexpr int VP = W + 1, ZP = W + 2;  // row pitches of a tile's values and planes
-    static constexpr int TILE = 32 * VP * 8 + 32 * ZP * 2;
-    __host__ __device__ static int cnt_at(int band) { return band * 16; }
-    __host__ __device__ static int touched_at(int band) { return cnt_at(band) + ((band * 2 + 15) & ~15); }
-    __host__ __device__ static int pitch(int band) {
-        return ((touched_at(band) + ((band * 2 + 15) & ~15) - 16 + 127) & ~127) + 16;
-    }
-    __host__ __device__ static size_t bytes(int band, int n) {
-        return (size_t)W * pitch(band) + 2 * TILE + (size_t)n * sizeof(Listed);
-    }
-};
-
-template <int W>
 __global__ void __launch_bounds__(W * 32, W == 8 ? 6 : 2)
 k_gather(const float2* __restrict__ rec, const int16_t* __restrict__ recz, const int2* __restrict__ posspec, int M,
          Params p, float2* __restrict__ vol, uint32_t* __restrict__ cnt_out, uint8_t* __restrict__ otf,
@@ -353,6 +327,7 @@ k_gather(const float2* __restrict__ rec, const int16_t* __restrict__ recz, const
     using S = GatherSmem<W>;
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ unsigned s_bal[2][32];
+    static_assert(sizeof(s_bal) == S::STATIC, "the form's choice counts it");
     const int band = p.band, F = p.F, D = p.D, h = D / 2, zmin = p.zmin;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int pitch = S::pitch(band), cnt_at = S::cnt_at(band);
@@ -816,7 +791,6 @@ int launch_gather_as(tdm_ctx* c, CapRecs rec, const int2* posspec, int n, uint32
                      cudaStream_t st) {
     const Params& p = c->p;
     const size_t smem = GatherSmem<W>::bytes(p.band, n);
-    if (smem > kMaxSmemPerCta) return TDM_EUNSUPPORTED;
     if (allow_smem(k_gather<W>, smem)) return TDM_ECUDA;
     Launch l(c, K_GATHER, st);
     k_gather<W><<<dim3((p.xb - p.xa) / W, p.yb - p.ya), W * 32, smem, st>>>(rec.val, rec.z, posspec, n, p, c->b.vol,
@@ -825,9 +799,11 @@ int launch_gather_as(tdm_ctx* c, CapRecs rec, const int2* posspec, int n, uint32
 }
 int launch_gather(tdm_ctx* c, CapRecs rec, const int2* posspec, int n, uint32_t* cnt, uint8_t* otf, int normalize,
                   cudaStream_t st) {
-    if (cnt && c->p.D >= 512 && GatherSmem<16>::bytes(c->p.band, n) <= kMaxSmemPerCta)
-        return launch_gather_as<16>(c, rec, posspec, n, cnt, otf, normalize, st);
-    return launch_gather_as<8>(c, rec, posspec, n, cnt, otf, normalize, st);
+    switch (gather_columns(c->p.D, c->p.band, n, cnt != nullptr)) {
+        case 16: return launch_gather_as<16>(c, rec, posspec, n, cnt, otf, normalize, st);
+        case 8: return launch_gather_as<8>(c, rec, posspec, n, cnt, otf, normalize, st);
+        default: return TDM_EUNSUPPORTED;
+    }
 }
 
 // x and y passes on the band planes, after the gather (DIR +1).
@@ -967,19 +943,6 @@ int adjoint_impl(tdm_ctx* c, CapRecs recs, int n, float* xn, float* xk, bool nor
 
 }  // namespace
 
-// The angle limit of a context: an angle count is accepted while a list of
-// 8-byte entries fits a CTA's shared memory beside the FP64 sums and counts of
-// four warps' columns (two columns a warp up to D = 512, whose FFT takes half a
-// warp), or their FFT exchange buffers, the plane owners, a staging row and
-// the mask bits.  k_gather, with 4-byte entries, needs less for every band
-// (at most sqrt(2) F + 2 planes, F <= 512) and count that this accepts.
-size_t gather_limit_bytes(int D, int band, int n) {
-    const int T = D / warp_fft_e(D), G = 32 / T;
-    const size_t sums = (size_t)G * band * (sizeof(double2) + sizeof(uint16_t)), xch = (size_t)G * T * (T + 1) * sizeof(float2);
-    const size_t region = ((sums > xch ? sums : xch) + 15) & ~size_t(15);
-    return 4 * (region + 32 * sizeof(float2) + ((band + 15) & ~15)) + (((size_t)band * 4 + 7) & ~size_t(7)) +
-           (size_t)n * sizeof(int2);
-}
 int launch_cap(tdm_ctx* c, int a0, int n, bool form, const float2* fields_in) {
     if (c->p.F & (c->p.F - 1)) return launch_cap_generic(c, a0, n, form, fields_in);
     switch (c->p.F) {

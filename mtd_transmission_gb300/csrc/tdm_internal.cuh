@@ -9,6 +9,7 @@
 #include "../../include/tdm.h"
 #include "fft_core.cuh"
 #include "argmax.cuh"
+#include "gather_smem.cuh"
 
 namespace tdm {
 
@@ -166,10 +167,6 @@ struct tdm_ctx {
 
 // Kernel launchers (defined in the kernel translation units).
 namespace tdm {
-// Shared memory that sets a context's angle limit, for a cap band of `band`
-// planes and n angles (the gather keeps each CTA's list of angles there).
-size_t gather_limit_bytes(int D, int band, int n);
-constexpr size_t kMaxSmemPerCta = 227 * 1024;
 // Scope around one kernel launch on c->stream: counts the launch and, when
 // profiling is on, brackets it with a pair of CUDA events.
 cudaEvent_t prof_event(tdm_ctx* c);
