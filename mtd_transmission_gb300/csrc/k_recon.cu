@@ -31,6 +31,7 @@
 #include "fp_bits.cuh"
 #include "cap_geometry.cuh"
 #include "gather_smem.cuh"
+#include "quotient.cuh"
 
 namespace tdm {
 namespace {
@@ -295,13 +296,6 @@ __device__ __forceinline__ void gather_add(ColumnSums& c, int z, float2 v, const
     }
     c.hit += __popc(fresh);
     __syncwarp();
-}
-
-// x / n, correctly rounded, from r the correctly rounded 1 / n (Markstein's
-// quotient correction); infinities and NaN as the division gives them.
-__device__ __forceinline__ float over(float x, float n, float r) {
-    const float q = x * r, rest = fmaf(-q, n, x);
-    return rest == rest ? fmaf(rest, r, q) : q;
 }
 
 // k_gather: a CTA of W warps takes W consecutive columns at one Y.  Each warp

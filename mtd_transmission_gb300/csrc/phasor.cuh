@@ -2,6 +2,7 @@
 // the field and Volkov passes of both FFT engines (k_fields.cu, k_generic.cu).
 #pragma once
 
+#include "quotient.cuh"
 #include "tdm_internal.cuh"
 
 namespace tdm {
@@ -9,9 +10,9 @@ namespace tdm {
 constexpr float kInvTwoPi = 0.15915494309189535f;
 
 // Amplitude |u| and unit phasor u/|u| (1 where u = 0: atan2(0, 0) = 0) from one
-// reciprocal square root: |u|^2 r, corrected by a Newton step of the square
-// root, and u r.  A field value whose square leaves the normal range is scaled
-// first.
+// reciprocal square root r: |u|^2 r, corrected by one step of Newton's iteration
+// for the square root, and u r.  A field value whose square leaves the normal range
+// is scaled first, and its amplitude is hypotf's.
 __device__ __forceinline__ float amplitude(float2 u, float2& z) {
     auto unit = [&](float2 w) {
         const float m2 = fmaf(w.x, w.x, w.y * w.y), r = rsqrtf(m2), m = m2 * r;
@@ -45,13 +46,6 @@ enum FieldMode { FIELD, PHASE, VOLKOV, VOLKOV_PHASE };
 // fifth of the row pass: 100 angles of 256^2 32 -> 27 us).
 __device__ __forceinline__ float phasor_gradient(float2 g, float2 z) {
     return (g.y * z.x - g.x * z.y) * (2.0f - fmaf(z.x, z.x, z.y * z.y)) * kInvTwoPi;
-}
-
-// x / y for y well inside the normal range: an approximate reciprocal and one
-// correction of the quotient.
-__device__ __forceinline__ float quotient(float x, float y) {
-    const float r = __fdividef(1.0f, y), q = x * r;
-    return fmaf(fmaf(-q, y, x), r, q);
 }
 
 }  // namespace tdm
