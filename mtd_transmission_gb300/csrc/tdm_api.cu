@@ -377,6 +377,7 @@ int tdm_create(const tdm_geom* geom, int max_angles, tdm_ctx** out) {
         cudaEventCreateWithFlags(&c->ev_lane_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_angles, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_vol_last, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_capture_end, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_rec_free[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_rec_free[1], cudaEventDisableTiming) != cudaSuccess) {
         delete c;
@@ -501,7 +502,7 @@ int tdm_destroy(tdm_ctx* c) {
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     if (c->dl_stream) cudaStreamDestroy(c->dl_stream);
     if (c->vol_stream) cudaStreamDestroy(c->vol_stream);
-    for (cudaEvent_t e : {c->ev_angles, c->ev_vol_last, c->ev_rec_free[0], c->ev_rec_free[1], c->ev_lane_fork})
+    for (cudaEvent_t e : {c->ev_angles, c->ev_vol_last, c->ev_capture_end, c->ev_rec_free[0], c->ev_rec_free[1], c->ev_lane_fork})
         if (e) cudaEventDestroy(e);
     delete c;
     return TDM_OK;
@@ -972,12 +973,14 @@ static int pipeline(tdm_ctx* c, const void* holos, int bits, int n, float* indic
     }
     TDM_CU(cudaEventRecord(c->ev_angles, c->stream));
     TDM_CU(cudaStreamWaitEvent(c->vol_stream, c->ev_angles, 0));
+    // A capture's records are nodes of its graph: the events that order calls outside of it keep what they hold, and
+    // the capture ends joined through an event of its own.
     int rc = run_volume(c, n, false, indice_out, absorption_out, otf_out, counts_out, wait, c->vol_stream,
-                        &c->b.rec_buf[par], c->b.posspec_vol[par], c->ev_rec_free[par]);
+                        &c->b.rec_buf[par], c->b.posspec_vol[par], capturing ? nullptr : c->ev_rec_free[par]);
     if (rc) return rc;
-    TDM_CU(cudaEventRecord(c->ev_vol_last, c->vol_stream));
+    TDM_CU(cudaEventRecord(capturing ? c->ev_capture_end : c->ev_vol_last, c->vol_stream));
     c->rec_parity ^= 1;
-    if (capturing) TDM_CU(join_volume(c));  // a capture must end joined
+    if (capturing) TDM_CU(cudaStreamWaitEvent(c->stream, c->ev_capture_end, 0));
     if (posspec_out && !is_device_ptr(posspec_out)) {
         std::vector<int2> tmp(n);
         TDM_CU(cudaMemcpyAsync(tmp.data(), c->b.posspec, n * sizeof(int2), cudaMemcpyDeviceToHost, c->stream));

@@ -152,6 +152,7 @@ struct tdm_ctx {
     cudaEvent_t ev_lane_join[tdm::kMaxLanes - 1] = {};
     cudaEvent_t ev_angles = nullptr;     // per-angle stages of the current call done (stream)
     cudaEvent_t ev_vol_last = nullptr;   // last volume stage queued on vol_stream
+    cudaEvent_t ev_capture_end = nullptr;  // the volume stage of a call that is captured into a graph
     cudaEvent_t ev_rec_free[2] = {};     // gather that read rec_buf[i] done
     int rec_parity = 0;
     cudaEvent_t ev_copy[tdm::kStageSlots] = {};  // upload into hologram staging slot s done
