@@ -282,9 +282,13 @@ int tdm_set_wait_limit(tdm_ctx* ctx, long long polls);
 int tdm_set_schedule(tdm_ctx* ctx, int chunk, int lanes);
 
 /* Project autotuner (no counterpart in the reference): times tdm_pipeline on
- * the given stack (device holograms) with the schedules (chunk, lanes) = (16, 4),
- * (16, 2), (8, 4), (12, 4), (32, 2), (16, 6) and (32, 4) that fit the context's
- * scratch and keeps the fastest; *chunk_out receives its chunk. */
+ * the given stack (device holograms) with the context's present schedule, its
+ * default one and those of (chunk, lanes) = (16, 4), (16, 2), (8, 4), (12, 4),
+ * (32, 2), (16, 6) and (32, 4) that fit the context's scratch, and keeps the fastest
+ * for holograms in device memory (the schedule for host holograms, which the
+ * uploads bound, stays).  *chunk_out receives the chunk of the fastest of the
+ * listed seven, or the present one where none fits.  After an error the
+ * context has the schedule that it had. */
 int tdm_autotune(tdm_ctx* ctx, const void* holos, int bits, int n, int* chunk_out);
 
 /* Stream-ordered execution helpers.  tdm_pipeline queues each volume's stage

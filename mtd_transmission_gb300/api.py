@@ -319,7 +319,8 @@ class Context:
         self._check(lib().tdm_set_wait_limit(self._h, polls), "tdm_set_wait_limit")
 
     def autotune(self, holos, n=None) -> int:
-        """tdm_autotune: picks the fastest schedule (chunk, lanes) on this stack; returns its chunk."""
+        """tdm_autotune: keeps the fastest schedule (chunk, lanes) on this stack, the present one included; returns
+        the chunk of the fastest of the listed ones."""
         n = holos.shape[0] if n is None else n
         out = ctypes.c_int()
         self._check(lib().tdm_autotune(self._h, ptr(holos), self._bits(holos), n, ctypes.byref(out)), "tdm_autotune")

@@ -201,6 +201,26 @@ int build_aberration(tdm_ctx* c, const uint8_t* mask_host) {
     return TDM_OK;
 }
 
+// Default schedule of the pipeline's per-angle stages.  Holograms in host memory: four chunks in flight, so that the
+// uploads of later ones overlap, a quarter of the scratch each (200 x 512^2: (32, 4) 0.48, (16, 4) 0.65 ms a volume),
+// but no more angles in flight than leave the extraction's band, the largest hand-over between two kernels, in L2, and
+// no chunks of a few angles, whose launches cost more than they fill.
+// Holograms in device memory: fewer and larger launches, two chunks in flight, unless three chunks' bands can stay in
+// L2 where the whole scratch's cannot.  Nearly stay: up to 15 % over its 126 MB, since a chunk's band is not all
+// written when its first rows are read; 24 angles of 1024^2 are 144 MB, and fewer were not timed.  Volumes of one
+// context alone / of three contexts in turn without waiting, in us: 600 x 1024^2 (16, 4) 3400/3770, (64, 2) 3230/3900,
+// (24, 3) 3320/3450, (128, 1) 3550/3510 (alone two chunks are a little faster there, among others three clearly);
+// 64 x 2048^2 (16, 4) 8810/9100, (32, 2) 8810/8870; 200 x 512^2 (32, 4) 460/370, (64, 2) 450/360; 400 x 256^2 (32, 4)
+// 430/300, (64, 2) 400/190; 48 x 512^2 (24, 2) 287/174, (16, 3) 302/180; 48 x 256^2 (24, 2) 175/73, (16, 3) 197/94.
+Schedule default_schedule(const tdm_ctx* c, bool dev) {
+    const size_t band_bytes = (size_t)c->p.H * c->p.F * sizeof(float2);
+    if (!dev) return {std::max(16, std::min(c->chunk_cap, (int)(kL2Bytes / band_bytes)) / 4), 4};
+    const int three = (int)(kL2Bytes * 115 / 100 / (3 * band_bytes));
+    const bool keep = three >= 16 && (size_t)c->chunk_cap * band_bytes > kL2Bytes;
+    const int lanes = keep ? 3 : 2;
+    return {std::max(16, std::min(c->chunk_cap / lanes, keep ? three : c->chunk_cap)), lanes};
+}
+
 int check_geom(const tdm_geom* g, std::string& why) {
     if (!is_pow2(g->ccd_roix) || g->ccd_roix < 256 || g->ccd_roix > 2048) {
         why = "CCD_ROIX must be a power of two in [256, 2048]";
@@ -278,21 +298,8 @@ int tdm_create(const tdm_geom* geom, int max_angles, tdm_ctx** out) {
     p.rayon = c->dv.rayon;
     p.inv_rayon = 1.0 / c->dv.rayon;
     const int N = p.N, F = p.F, D = p.D;
-    // The pipeline's chunks.  Holograms in host memory: four in flight, so that the uploads of later ones overlap, a
-    // quarter of the scratch each (200 x 512^2: (32, 4) 0.48, (16, 4) 0.65 ms a volume), but no more angles in flight
-    // than leave the extraction's band, the largest hand-over between two kernels, in L2, and no chunks of a few
-    // angles, whose launches cost more than they fill.
-    const size_t band_bytes = (size_t)p.H * F * sizeof(float2);
-    c->chunk = c->holo_chunk = std::max(16, std::min(c->chunk_cap, (int)(kL2Bytes / band_bytes)) / c->lanes);
-    // Holograms in device memory: fewer and larger launches, two chunks in flight, unless three chunks' bands can
-    // stay (nearly) in L2 where the whole scratch's cannot.  Volumes of one context alone / of three contexts in turn
-    // without waiting, in us: 600 x 1024^2 (16, 4) 3400/3770, (64, 2) 3230/3900, (24, 3) 3320/3450, (128, 1)
-    // 3550/3510; 64 x 2048^2 (16, 4) 8810/9100, (32, 2) 8810/8870; 200 x 512^2 (32, 4) 460/370, (64, 2) 450/360;
-    // 400 x 256^2 (32, 4) 430/300, (64, 2) 400/190.
-    const int three = (int)(kL2Bytes * 115 / 100 / (3 * band_bytes));
-    const bool keep = three >= 16 && (size_t)c->chunk_cap * band_bytes > kL2Bytes;
-    c->dev_lanes = keep ? 3 : 2;
-    c->dev_chunk = std::max(16, std::min(c->chunk_cap / c->dev_lanes, keep ? three : c->chunk_cap));
+    c->holo = default_schedule(c, false);
+    c->dev = default_schedule(c, true);
     // disc test fd^2 < COEF_NA_OBJ_LIMIT * N^2 on integers (fonctions.cpp:915)
     const double lim = geom->coef_na_obj_limit * (double)(N * N);
     p.disc_thr = (int)std::min<double>(std::ceil(lim), 2.0 * N * N + 1);
@@ -649,13 +656,13 @@ double tdm_stage_ms(const tdm_ctx* c, const char* stage) {
 }
 
 // ---------------------------------------------------------------- stages
-// Hologram staging for host stacks: a ring of slots of holo_chunk holograms
+// Hologram staging for host stacks: a ring of slots of holo.chunk holograms
 // (16-bit size) in the 2 chunk_cap holograms of b.holo_stage.
 static int stage_slots(const tdm_ctx* c) {
-    return std::max(1, std::min(kStageSlots, 2 * c->chunk_cap / c->holo_chunk));
+    return std::max(1, std::min(kStageSlots, 2 * c->chunk_cap / c->holo.chunk));
 }
 static uint8_t* stage_slot(tdm_ctx* c, int s) {
-    return c->b.holo_stage + (size_t)s * c->holo_chunk * c->p.H * c->p.H * 2;
+    return c->b.holo_stage + (size_t)s * c->holo.chunk * c->p.H * c->p.H * 2;
 }
 // Chunks per hologram upload in the pipeline: up to 4 consecutive staging
 // slots take one copy (a divisor of the ring's slot count, and at most a
@@ -676,8 +683,8 @@ static int stage_extract(tdm_ctx* c, const void* holos, int bits, int n, float2*
     if (is_device_ptr(holos)) return launch_extract(c, holos, bits, n, 0, false, also);
     // host holograms: chunked copies on the copy stream into a ring of staging slots
     const int nslot = stage_slots(c);
-    for (int h0 = 0, k = 0; h0 < n; h0 += c->holo_chunk, ++k) {
-        const int m = std::min(c->holo_chunk, n - h0);
+    for (int h0 = 0, k = 0; h0 < n; h0 += c->holo.chunk, ++k) {
+        const int m = std::min(c->holo.chunk, n - h0);
         const int buf = k % nslot;
         uint8_t* dst = stage_slot(c, buf);
         TDM_CU(cudaStreamWaitEvent(c->copy_stream, c->ev_free[buf], 0));  // no-op before its first record
@@ -882,7 +889,7 @@ static int stage_angles(tdm_ctx* c, const void* holos, int bits, int n, int2* po
     const Params& p = c->p;
     const size_t per = (size_t)p.H * p.H * (bits == 16 ? 2 : 1);
     const bool dev = is_device_ptr(holos);
-    const int chunk = dev ? c->dev_chunk : c->holo_chunk, lanes = dev ? c->dev_lanes : c->lanes;
+    const auto [chunk, lanes] = dev ? c->dev : c->holo;
     const int nchunks = (n + chunk - 1) / chunk;
     const int nl = std::max(1, std::min(std::min(lanes, kMaxLanes), std::min(c->chunk_cap / chunk, nchunks)));
     const int nslot = stage_slots(c), grp = upload_group(nslot);
@@ -1229,8 +1236,7 @@ int tdm_set_schedule(tdm_ctx* c, int chunk, int lanes) {
         return fail(c, TDM_EINVAL, "tdm_set_schedule: need 1 <= lanes <= 8 and chunk * lanes <= the chunk capacity");
     cudaSetDevice(c->device);
     if (int rc = tdm_synchronize(c)) return rc;  // the staging ring's slots move with the chunk size
-    c->chunk = c->holo_chunk = c->dev_chunk = chunk;
-    c->lanes = c->dev_lanes = lanes;
+    c->holo = c->dev = {chunk, lanes};
     return TDM_OK;
 }
 
@@ -1239,15 +1245,18 @@ int tdm_autotune(tdm_ctx* c, const void* holos, int bits, int n, int* chunk_out)
         return fail(c, TDM_EINVAL, "tdm_autotune: invalid argument (device holograms required)");
     cudaSetDevice(c->device);
     if (int rc = tdm_synchronize(c)) return rc;
-    const int cands[][2] = {{16, 4}, {16, 2}, {8, 4}, {12, 4}, {32, 2}, {16, 6}, {32, 4}};
-    int best = c->dev_chunk, best_lanes = c->dev_lanes;
-    float best_ms = 0;
+    // the context's own schedule first: it stays unless another one is faster
+    const Schedule before = c->dev, usual = default_schedule(c, true);
+    const Schedule tried[] = {before, usual, {16, 4}, {16, 2}, {8, 4}, {12, 4}, {32, 2}, {16, 6}, {32, 4}};
+    constexpr int kListed = 2;  // the listed ones, whose fastest chunk_out names, start here
+    Schedule best = before, listed = before;
+    float best_ms = 0, listed_ms = 0;
     cudaEvent_t t0 = prof_event(c), t1 = prof_event(c);
     int rc = TDM_OK;
-    for (const auto& cand : cands) {
-        if (cand[0] * cand[1] > c->chunk_cap) continue;
-        c->dev_chunk = cand[0];
-        c->dev_lanes = cand[1];
+    for (int i = 0; i < (int)(sizeof(tried) / sizeof(tried[0])); ++i) {
+        const Schedule k = tried[i];
+        if (i >= kListed ? k.chunk * k.lanes > c->chunk_cap : i && k == before) continue;
+        c->dev = k;
         rc = pipeline(c, holos, bits, n, nullptr, nullptr, nullptr, nullptr, nullptr, false);  // warm-up
         if (!rc && cudaEventRecord(t0, c->stream) != cudaSuccess) rc = TDM_ECUDA;
         for (int r = 0; r < 2 && !rc; ++r) rc = pipeline(c, holos, bits, n, nullptr, nullptr, nullptr, nullptr, nullptr, false);
@@ -1256,18 +1265,14 @@ int tdm_autotune(tdm_ctx* c, const void* holos, int bits, int n, int* chunk_out)
         float ms = 0;
         if (!rc && cudaEventElapsedTime(&ms, t0, t1) != cudaSuccess) rc = TDM_ECUDA;
         if (rc) break;
-        if (best_ms == 0 || ms < best_ms) {
-            best_ms = ms;
-            best = cand[0];
-            best_lanes = cand[1];
-        }
+        if (best_ms == 0 || ms < best_ms) best_ms = ms, best = k;
+        if (i >= kListed && (listed_ms == 0 || ms < listed_ms)) listed_ms = ms, listed = k;
     }
     c->ev_pool.push_back(t0);
     c->ev_pool.push_back(t1);
-    c->chunk = c->holo_chunk = c->dev_chunk = best;
-    c->lanes = c->dev_lanes = best_lanes;
+    c->dev = rc ? before : best;
     if (rc) return rc;
-    if (chunk_out) *chunk_out = best;
+    if (chunk_out) *chunk_out = listed.chunk;
     return TDM_OK;
 }
 

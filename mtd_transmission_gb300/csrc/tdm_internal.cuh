@@ -108,6 +108,13 @@ enum KernelId {
 };
 extern const char* const kKernelNames[K_COUNT];
 
+// Schedule of the pipeline's per-angle stages (tdm_set_schedule, tdm_autotune): angles per chunk, and chunks in flight at
+// once, as far as lanes * chunk <= chunk_cap.
+struct Schedule {
+    int chunk, lanes;
+    bool operator==(const Schedule& o) const { return chunk == o.chunk && lanes == o.lanes; }
+};
+
 struct ProfRec {
     int id;
     cudaEvent_t a, b;
@@ -121,10 +128,7 @@ struct tdm_ctx {
     tdm::Params p{};
     tdm::Buffers b{};
     int max_angles = 0;
-    int chunk = 16;              // angles per chunk of the pipeline's per-angle stages (tdm_set_schedule, tdm_autotune)
-    int holo_chunk = 16;         // holograms per extraction chunk (equal to chunk)
-    int lanes = 4;               // chunks in flight at once; lanes * chunk <= chunk_cap
-    int dev_chunk = 16, dev_lanes = 4;  // the same for holograms in device memory
+    tdm::Schedule holo{16, 4}, dev{16, 4};  // the pipeline's schedules for holograms in host and in device memory
     int chunk_cap = 64;          // angles of per-chunk scratch: min(128, max_angles rounded up to 16)
     int nsamp = 0;
     int device = 0;
