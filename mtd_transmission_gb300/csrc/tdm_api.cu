@@ -725,8 +725,12 @@ static int run_fields(tdm_ctx* c, const float* spectra_in, int n, float* fields_
     const size_t FF = (size_t)c->p.F * c->p.F;
     FieldIo io;
     if (c->p.c_aber && is_direct(c, fields_out)) io.fields = reinterpret_cast<float2*>(fields_out);
-    if (is_direct(c, spectra_in) &&
-        !(io.fields && overlap(spectra_in, n * FF * sizeof(float2), fields_out, n * FF * sizeof(float2))))
+    // outputs that are written launch by launch, while later launches' spectra are unread
+    auto over_spectra = [&](const void* out, size_t pixel) {
+        return out && overlap(spectra_in, n * FF * sizeof(float2), out, n * FF * pixel);
+    };
+    if (is_direct(c, spectra_in) && !over_spectra(io.fields, sizeof(float2)) && !over_spectra(dph, sizeof(float)) &&
+        !over_spectra(dun, sizeof(float)) && !over_spectra(dam, sizeof(float)))
         io.spectra = reinterpret_cast<const float2*>(spectra_in);
     if (spectra_in && !io.spectra && spectra_in != reinterpret_cast<float*>(c->b.spectra)) {
         TDM_CU(cudaMemcpyAsync(c->b.spectra, spectra_in, n * FF * sizeof(float2), cudaMemcpyDefault, c->stream));
