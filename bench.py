@@ -50,7 +50,8 @@ def algorithmic_bytes(name, acq, hits_per_angle, band):
         "extract_cols": H * F * 8 + F * F * 8,
         "argmax": F * F * 8,
         "field_rows": F * F * 8 * 2,
-        "field_cols": F * F * 8 + F * F * 4 * 2,
+        # the field's rows in, amplitude and unit phasor out
+        "field_cols": F * F * 8 + F * F * (4 + 8),
         # phasor in, gx out
         "volkov_rows": F * F * 8 + F * F * 4,
         # phasor and gx in; the columns' DCT-II of gx and DST-II of gy out
@@ -130,23 +131,18 @@ def stage_roofline(acq, hits_per_angle, kern_ms, step_ms, peak):
     return out
 
 
-# DRAM bytes (read + write) per launch from the committed ncu capture of
-# the kernel on this code (the file named in the returned source), as
-# (bytes that do not depend on the angle count, bytes per 600 angles): the
-# row pass on the 64-hologram case (a launch processes 16 holograms), the
-# gather on the 600-angle workload (its record reads grow with the angles;
-# its volume and OTF writes do not).  None where no capture of this
-# workload's kernel is committed.
+# DRAM bytes (read + write) per launch from a committed ncu capture (the file
+# named beside them): the hologram row pass of a launch of 16 holograms of
+# 1024^2.  None where no capture of this workload's kernel is committed.
 NCU_TRAFFIC = {
-    "extract_rows": (33.616128e6 + 0.341504e6, 0.0, "profiles/k_extract_rows_rytov_1024_64holos.md"),
+    "extract_rows": (33.602560e6 + 0.185088e6, "profiles/kernels_64_angles.md"),
 }
 
 
 def ncu_traffic_per_launch(name, acq):
-    if acq.ccd_roix != 1024 or acq.nxmax != 128 or acq.dim_final != 512 or name not in NCU_TRAFFIC:
+    if acq.ccd_roix != 1024 or acq.nxmax != 128 or acq.dim_final != 512:
         return None, None
-    fixed, per600, src = NCU_TRAFFIC[name]
-    return fixed + per600 * acq.nb_holo / 600, src
+    return NCU_TRAFFIC.get(name, (None, None))
 
 
 def measured_peaks():

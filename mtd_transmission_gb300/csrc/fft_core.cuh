@@ -49,7 +49,8 @@ __device__ __forceinline__ float2 c_conj(float2 a) { return make_float2(a.x, -a.
 // part is not exactly 0, a transform's value is 0 by accident in 1 of 1e8 cells,
 // and after any change of rounding in other cells.  So the first sums of a
 // butterfly, the only ones that products reach, are scalar for this type; the rest is
-// packed.  (600 x 1024^2 to 512^3 3398 us, with packed first sums 3399.  The
+// packed.  Which of them the compiler fuses is its own choice (nvcc 13.0, -fmad on), so
+// another compiler may set such a cell's mark differently.  (600 x 1024^2 to 512^3 3398 us, with packed first sums 3399.  The
 // mixed-radix butterflies take their products through fma() or shared memory and
 // need no such type; all scalar they took 500 x 250^2 to 512^3 from 1450 to 1555 us.)
 struct alignas(8) Fusable {

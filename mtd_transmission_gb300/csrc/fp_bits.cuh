@@ -3,10 +3,12 @@
 // The GB300 FP64 pipe runs at a small fraction of the FP32 rate and the
 // hardware conversions between float and double issue on it.  The misfit of the
 // forward operator squares and adds FP32 residuals in FP64; widening them on the
-// integer pipe leaves the FP64 pipe to that.  Both functions give the exact IEEE
+// integer pipe leaves the FP64 pipe to that.  Both directions give the exact IEEE
 // results: widening is exact, narrowing rounds to nearest, ties to even, with
 // subnormal results, overflow to infinity and NaN handled as the standard
-// says.  The header also compiles as plain C++ for the host-side check.
+// says.  No kernel narrows at present (the cap sums, pairs of floats, need no
+// FP64); narrow() is widen()'s counterpart in the host-side check, for which the
+// header also compiles as plain C++.
 #pragma once
 
 #include <cstdint>

@@ -71,10 +71,11 @@ __global__ void __launch_bounds__(256) k_argmax_part(const float2* __restrict__ 
 }
 
 // ---------------------------------------------------------------- field = shift(IFFT(shift(S)))
-// All FFT passes below run on the warp-resident FFT (fft_warp.cuh).  A row
-// pass loads and stores its lanes' elements directly (lane-minor order is
-// contiguous along a row); a column pass stages B columns in shared memory
-// with CTA-wide coalesced loads and stores around the transforms.
+// The row passes below run on the warp-resident FFT (fft_warp.cuh): a warp's
+// lanes load and store their elements directly (lane-minor order is contiguous
+// along a row).  In the column passes the lanes run across columns (ColFFT), so
+// that their loads and stores are whole pieces of rows; shared memory holds the
+// transforms' exchanges only.
 template <int F>
 struct FieldCfg {
     using W = WarpFFT<F>;

@@ -310,7 +310,8 @@ __device__ __forceinline__ void gather_add(ColumnSums& c, int z, float2 v, const
 // angles of 256^2 to 512^3 418 -> 381 us, 64 of 512^2 to 1024^3 3.5 -> 2.3 ms; at
 // 256^3 8 columns take 76 us, 16 90).
 //
-// Bound by issue and latency.  600 angles of 256^2 to 512^3: 434 us (with FP64
+// Bound by issue and latency (64 angles, 8 columns a CTA: issue 77 % active at 59 % of
+// the warps; six CTAs an SM leave 40 registers, and 20 bytes are spilled).  600 angles of 256^2 to 512^3: 434 us (with FP64
 // sums of FP32 group sums, and each lane loading its angle's records, 538); 400
 // of 128^2 to 256^3 76 us (100).
 template <int W>
@@ -557,7 +558,8 @@ k_fzpass(const float* __restrict__ re, const float* __restrict__ im, const float
 // Cap values of the spectrum: for each angle and FFT bin, the spectrum at its
 // cap cell (0 outside the cap).  With data (cap values of measurements), the
 // residual spectrum - data on the cap cells (0 elsewhere) and the misfit
-// sum |residual|^2 added to *misfit.
+// sum |residual|^2 added to *misfit.  (8 bytes are spilled around the call that
+// computes a height outside the table, which caps inside the field do not make.)
 __global__ void __launch_bounds__(256)
 k_cap_sample(const float2* __restrict__ vol, const int2* __restrict__ posspec, Params p,
              const double* __restrict__ s_tab, const float2* __restrict__ s_pair, const float2* __restrict__ data,

@@ -206,10 +206,11 @@ int build_aberration(tdm_ctx* c, const uint8_t* mask_host) {
 // but no more angles in flight than leave the extraction's band, the largest hand-over between two kernels, in L2, and
 // no chunks of a few angles, whose launches cost more than they fill.
 // Holograms in device memory: fewer and larger launches, two chunks in flight, unless three chunks' bands can stay in
-// L2 where the whole scratch's cannot.  Nearly stay: up to 15 % over its 126 MB, since a chunk's band is not all
-// written when its first rows are read; 24 angles of 1024^2 are 144 MB, and fewer were not timed.  Volumes of one
-// context alone / of three contexts in turn without waiting, in us: 600 x 1024^2 (16, 4) 3400/3770, (64, 2) 3230/3900,
-// (24, 3) 3320/3450, (128, 1) 3550/3510 (alone two chunks are a little faster there, among others three clearly);
+// L2, or exceed its 126 MB by no more than 15 %, where the whole scratch's cannot.  Volumes of one context alone / of
+// three contexts in turn without waiting, in us: 600 x 1024^2 (16, 4) 3400/3770, (64, 2) 3230/3900, (24, 3) 3320/3450,
+// (128, 1) 3550/3510 (alone two chunks are a little faster there, among others three clearly); three chunks of other
+// sizes (another run, with (64, 2) 3188/3757) 16: 3516/3351, 20: 3407/3340, 24: 3312/3343, 26: 3265/3382, 28:
+// 3296/3685, 42: 3166/3553, so the 15 % end before the rise at 28;
 // 64 x 2048^2 (16, 4) 8810/9100, (32, 2) 8810/8870; 200 x 512^2 (32, 4) 460/370, (64, 2) 450/360; 400 x 256^2 (32, 4)
 // 430/300, (64, 2) 400/190; 48 x 512^2 (24, 2) 287/174, (16, 3) 302/180; 48 x 256^2 (24, 2) 175/73, (16, 3) 197/94.
 Schedule default_schedule(const tdm_ctx* c, bool dev) {

@@ -144,7 +144,7 @@ struct tdm_ctx {
     // downloads of the staged outputs done, per part (index, absorption, counts, OTF): a volume
     // stage waits for the previous volume's download of a part just before it rewrites that part
     cudaEvent_t ev_dl[tdm::kOutEvents] = {};
-    // tdm_pipeline runs each volume's stage (gather, z/y/x passes) on vol_stream, so that it
+    // tdm_pipeline runs each volume's stage (gather, x/y/z passes) on vol_stream, so that it
     // overlaps the next call's per-angle stages; the cap records and the specular positions the
     // volume stage reads are double buffered
     cudaStream_t vol_stream = nullptr;
